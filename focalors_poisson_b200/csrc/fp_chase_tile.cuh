@@ -1,0 +1,224 @@
+// One-pass partition chase: the Thomas solves along x of W neighbouring wavenumbers by one CTA that holds all
+// their rows in registers, so that a field is read once and written once.
+//
+// Rows are cut into P chunks, the first e of R rows and the others of R - 1 (so any nx but a few below 13 divides,
+// tile_rows), thread (p, w) = (threadIdx.x / W, threadIdx.x % W) owns chunk p of wavenumber j = tile W + w. The last row of a chunk
+// is its separator B_p; the rows before it satisfy  x_int = z_p - B_{p-1} g - B_p h,  z_p = T^-1 f_int,
+// g = T^-1 e_first, h = T^-1 e_last, and the separators a tridiagonal system of size P whose Thomas factors
+// depend on the wavenumber only and are tabulated:
+//   -g_last B_{p-1} + (d - h_last - g'_first) B_p - h'_first B_{p+1} = f_sep - z_last - z'_first
+// (primes: the next chunk). A pass: the forward elimination of every chunk (its values stay in registers), z_first
+// by a back substitution that stores nothing; the separator system as two affine scans along p (shuffles inside a
+// warp, the warps' compositions through shared memory); then the elimination's values are corrected by B_{p-1} and
+// substituted back from B_p. The Thomas factors c of one chunk serve every sweep and come from shared memory.
+// Periodic x: the last row is a cut, beta = x_{nx-1}. The other separators are solved for beta = 0, the wrapped
+// row gives beta, and their response v to beta = 1 (tabulated) is added.
+// The result equals the sequential Thomas solve (chasing_method_base.cpp:24-52) and, for periodic x, the
+// Sherman-Morrison solve (:178-197) up to round-off.
+//
+// What bounds it: one read and one write of the field (L2 or HBM); 2048 x 2048 in 27.5 us, 2.4 TB/s (the three-pass
+// form: 48 us), 256 x 65536 in 79 us, 3.4 TB/s; the load, compute and store phases of the few tiles an SM holds
+// overlap little. At R = 16 the kernel stays at 64 registers, so
+// that an SM holds 1024 threads of tiles, and the dependent chains at 15 steps. Only the last interior row of a
+// chunk is conditional: with a bound on every row the selects took 5/6 of the instructions.
+#pragma once
+
+#include "fp_common.cuh"
+
+namespace fpb
+{
+
+constexpr int kTileThreads = 1024;  // largest CTA: kTileThreads / 4 chunks
+constexpr int kTileMaxRows = kTileThreads / 4 * 16;
+
+// Rows of the longer chunks for nx rows, whose chunks of R and R - 1 rows must add up to nx; 0 where none does (nx = 2
+// and 5) or nx is beyond one CTA. 16 above 512 rows; 8 below, where a field gives few tiles and the pass is a chain
+// of latencies (graph replays, 128 x 128 / 384 x 384 / 96 x 11520 periodic: 3.2 / 4.0 / 5.8 us against 4.8 / 4.4 /
+// 8.3 us at R = 16; 2048 x 2048: 34.8 us against 27.5 us).
+inline int tile_rows(int nx)
+{
+    if (nx > kTileMaxRows) return 0;
+    for (int R : {16, 8, 4})
+        if ((R < 16 || nx > 512) && (nx + R - 1) / R * (R - 1) <= nx) return R;
+    return 0;
+}
+
+// The systems of one field: chunk layout and tables (chase_tile_tables builds them).
+struct ChaseTileTab
+{
+    int           nx, ny;      // rows; wavenumbers of a row
+    int           R, P, e;     // rows of a long chunk; chunks; the leading ones that are long
+    int           end_neu;     // x+ Neumann: the last row's diagonal is d + 1
+    int           per;         // periodic x
+    const double* cc;          // [2][R - 1][ny] Thomas factors: first chunk (x- Neumann change), others
+    const double* ends;        // [3][4][ny] g_first, g_last, h_first, h_last: chunk 0, other long ones, short ones
+    const double* d;           // [ny] diagonals
+    const double* cp;          // [P][ny] separator Thomas factors; the last row is formed in the kernel
+    const double* iden;        // [P][ny] 1 / denominators
+    const double* v;           // periodic: [P][ny] separators' response to beta = 1
+    const double* ib;          // periodic: [ny] 1 / the wrapped row's denominator
+};
+
+// Shared memory (doubles) of a CTA of n threads with tiles of W wavenumbers.
+__host__ __device__ __forceinline__ int chase_tile_smem(int n, int W, int R)
+{
+    return 2 * (R - 1) * W + 2 * n + 4 * (n / 32) * W + W;
+}
+
+// Inclusive affine scan over the chunks a warp holds (lane stride W), then over the CTA's warps: (a, b) of the
+// thread's own map becomes the value of the composition of every map before and including it, applied to 0.
+// REV: from the last chunk down. ta / tb: the warps' compositions, nw x W each. Contains one barrier.
+template <int W, bool REV>
+__device__ __forceinline__ double tile_scan(double a, double b, double* ta, double* tb)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, w = lane % W;
+    // W = 32: a warp holds one chunk
+#pragma unroll
+    for (int o = W; o < 32; o <<= 1)
+    {
+        const double pa = REV ? __shfl_down_sync(0xffffffffu, a, o) : __shfl_up_sync(0xffffffffu, a, o);
+        const double pb = REV ? __shfl_down_sync(0xffffffffu, b, o) : __shfl_up_sync(0xffffffffu, b, o);
+        if (REV ? lane + o < 32 : lane >= o)
+        {
+            b = fma(a, pb, b);
+            a *= pa;
+        }
+    }
+    if (REV ? lane < W : lane >= 32 - W)
+    {
+        ta[wid * W + w] = a;
+        tb[wid * W + w] = b;
+    }
+    __syncthreads();
+    double y = 0;
+    if (REV)
+        for (int v = nw - 1; v > wid; --v) y = fma(ta[v * W + w], y, tb[v * W + w]);
+    else
+        for (int v = 0; v < wid; ++v) y = fma(ta[v * W + w], y, tb[v * W + w]);
+    return fma(a, y, b);
+}
+
+// One tile. IO: in(i, j) the address of a right-hand side (rows ny apart), rhs(i, j, v) the value from what is
+// there, put(o, i, j, x, on) takes the solution for address o = out(i, j) (called by all
+// threads of a warp together, `on` where there is one). skip: wavenumbers from ny - skip on are left alone. The tile's
+// wavenumbers are tile W .. tile W + W - 1; blockDim.x a multiple of 32 of at least P W.
+template <int W, int R, typename IO>
+__device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int skip, const IO& io, double* sm)
+{
+    constexpr int Ri  = R - 1;
+    const int     n   = blockDim.x, tid = threadIdx.x;
+    const int     w   = tid % W, p = tid / W, P = t.P, ny = t.ny;
+    const int     j0  = tile * W + w;
+    const bool    act = p < P && j0 < ny - skip;
+    const int     j   = j0 < ny ? j0 : 0;  // idle lanes read column 0 and store nothing
+    double*       cs  = sm;                      // [2][Ri][W]
+    double*       zf  = cs + 2 * Ri * W;         // [n] first interior values; later the separators
+    double*       xs  = zf + n;                  // [n]
+    double*       ta  = xs + n;                  // warps' compositions, forward and backward
+    double*       tb  = ta + (n / 32) * W;
+    double*       ta2 = tb + (n / 32) * W;
+    double*       tb2 = ta2 + (n / 32) * W;
+    double*       sb  = tb2 + (n / 32) * W;      // [W] beta
+    const int     pc  = p < P ? p : P - 1;
+    const int     i0  = pc * (R - 1) + min(pc, t.e);
+    const bool    lng = pc < t.e;
+    const int     li  = lng ? Ri : Ri - 1;  // interior rows; idle threads repeat the last chunk
+
+    double y[Ri];
+    auto   pin = io.in(i0, j);
+#pragma unroll
+    for (int r = 0; r < Ri; ++r, pin += ny) y[r] = r < Ri - 1 || lng ? (double)*pin : 0.0;
+    double fsep = (double)*io.in(i0 + li, j);
+#pragma unroll
+    for (int r = 0; r < Ri; ++r)
+        if (r < Ri - 1 || lng) y[r] = io.rhs(i0 + r, j, y[r]);
+    fsep = io.rhs(i0 + li, j, fsep);
+#pragma unroll 4
+    for (int k = tid; k < 2 * Ri * W; k += n)
+        cs[k] = __ldg(t.cc + (long long)(k / W) * ny + min(tile * W + k % W, ny - 1));
+    // separator row of chunk p (the factors of the last row depend on its being last)
+    double        inv = 0, cpv = 0, gl = 0;
+    const double* en  = t.ends + (long long)(p == 0 ? 0 : p < t.e ? 1 : 2) * 4 * ny + j;
+    if (p < P)
+    {
+        gl = __ldg(en + ny);
+        if (p < P - 1)
+        {
+            inv = __ldg(t.iden + (long long)p * ny + j);
+            cpv = __ldg(t.cp + (long long)p * ny + j);
+        }
+        else if (!t.per)
+        {
+            const double diag = (t.end_neu ? __ldg(t.d + j) + 1.0 : __ldg(t.d + j)) - __ldg(en + 3 * (long long)ny);
+            inv = 1.0 / (p > 0 ? fma(gl, __ldg(t.cp + (long long)(p - 1) * ny + j), diag) : diag);
+        }
+    }
+    __syncthreads();
+
+    const double* c  = cs + (p == 0 ? 0 : Ri * W) + w;
+    double        zl = 0, z = 0;
+#pragma unroll
+    for (int r = 0; r < Ri; ++r)
+        if (r < Ri - 1 || lng)
+        {
+            zl   = (y[r] - zl) * c[r * W];
+            y[r] = zl;
+        }
+#pragma unroll
+    for (int r = Ri - 1; r >= 0; --r)
+        if (r < Ri - 1 || lng) z = fma(-c[r * W], z, y[r]);
+    zf[tid] = z;
+    __syncthreads();
+
+    const bool   sep = p < P - (t.per ? 1 : 0);  // rows of the separator system (the periodic cut is none of them)
+    double       rhs = fsep - zl;
+    if (p < P - 1) rhs -= zf[tid + W];
+    double x = tile_scan<W, false>(sep ? (p > 0 ? gl * inv : 0.0) : 1.0, sep ? rhs * inv : 0.0, ta, tb);
+    x        = tile_scan<W, true>(sep ? -cpv : 1.0, sep ? x : 0.0, ta2, tb2);
+    double bl;
+    if (t.per)
+    {
+        xs[tid] = x;
+        __syncthreads();
+        if (p == P - 1)
+        {
+            double num = fsep - zl - zf[w];
+            if (P > 1) num += gl * xs[tid - W] + __ldg(t.ends + 2 * (long long)ny + j) * xs[w];
+            sb[w] = num * __ldg(t.ib + j);
+        }
+        __syncthreads();
+        const double beta = sb[w];
+        x                 = p < P - 1 ? fma(__ldg(t.v + (long long)p * ny + j), beta, x) : beta;
+        zf[tid]           = x;
+        __syncthreads();
+        bl = p > 0 ? zf[tid - W] : beta;
+    }
+    else
+    {
+        xs[tid] = x;
+        __syncthreads();
+        bl = p > 0 ? xs[tid - W] : 0.0;
+    }
+
+    double dl = -bl;
+#pragma unroll
+    for (int r = 0; r < Ri; ++r)
+        if (r < Ri - 1 || lng)
+        {
+            dl *= r ? -c[r * W] : c[0];
+            y[r] += dl;
+        }
+    io.put(io.out(i0 + li, j), i0 + li, j, x, act);
+    auto po = io.out(i0 + Ri - 1, j);
+#pragma unroll
+    for (int r = Ri - 1; r >= 0; --r, po -= ny)
+    {
+        if (r < Ri - 1 || lng) x = fma(-c[r * W], x, y[r]);
+        io.put(po, i0 + r, j, x, r < Ri - 1 ? act : act && lng);
+    }
+}
+
+// `batch` fields of t.nx x t.ny values back to back, solved in place; wavenumbers from ny - skip on are left alone.
+void launch_chase_tile(double* f, long long batch, int skip, const ChaseTileTab& t, cudaStream_t s);
+
+}  // namespace fpb

@@ -175,6 +175,9 @@ template <typename T> struct DevRect
     DevBuf                           cc, cg, chh, cends, dsep;  // partition chase tables
     DevBuf                           sep_cp, sep_iden;          // separator-system Thomas factors [p][j]
     int                              sep_pmax = 0;              // rows of those tables
+    bool                             tiled    = false;          // one-pass chase (fp_chase_tile.cuh): FP64, nx <= 4096
+    int                              tile_R = 0, tile_P = 0, tile_e = 0;  // its chunks
+    DevBuf                           tile_cc, tile_ends, tile_d, tile_cp, tile_iden, tile_v, tile_ib;
     mutable DevBuf                   scratch;                   // partition chase scratch (per batch)
 
     // sep_rows: separator-factor rows to tabulate (default nx / 32; larger for tables shared by a batch)
@@ -190,7 +193,9 @@ template <typename T> struct DevRect
     // reduced-precision inner solve of iterative refinement. The FP32 transform plan is built on first use.
     void solve_mixed(T* f, long long batch, cudaStream_t s) const;
     mutable std::unique_ptr<DevTransform<float>> tr32;
-    // Scratch elements the partition chase needs for `batch` fields (0 when it is not used).
+    // Scratch elements the three-pass partition chase would take for `batch` fields (0 where it does not apply).
+    long long partition_elems(long long batch) const;
+    // Scratch elements the chase needs for `batch` fields.
     long long chase_scratch_elems(long long batch) const;
     // The chase alone, with caller-provided scratch of chase_scratch_elems(batch) elements.
     void chase(T* f, long long batch, T* scratch, cudaStream_t s) const;

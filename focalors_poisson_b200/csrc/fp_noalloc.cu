@@ -51,7 +51,7 @@ extern "C" int fp_rect_solve_f64_noalloc(fp_rect* r, double* f, long long batch,
         if (!f) throw fpb::Error(FP_ERR_INVALID, "null field pointer");
         if (batch < 0) throw fpb::Error(FP_ERR_INVALID, "negative batch");
         const fpb::DevRect<double>& plan = *r->r64;
-        const long long             need = plan.chase_scratch_elems(batch);
+        const long long             need = plan.partition_elems(batch);  // the documented limit, whatever chase runs
         if (need > kNoallocScratchDoubles)
             throw fpb::Error(FP_ERR_UNSUPPORTED,
                              "fp_rect_solve_f64_noalloc: this solve needs " + std::to_string(need) +

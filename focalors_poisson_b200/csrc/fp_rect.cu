@@ -1,5 +1,6 @@
 // Device-resident transform and rectangle (PoissonSolver2D) plans.
 #include "fp_chase.cuh"
+#include "fp_chase_tile.cuh"
 #include "fp_internal.h"
 
 #include <algorithm>
@@ -354,6 +355,91 @@ void separator_factors(int ny, int pmax, const std::vector<double>& d, const std
     }
 }
 
+namespace
+{
+// Tables of the one-pass chase (fp_chase_tile.cuh) for nx rows with diagonals d, R = tile_rows(nx). per: periodic x,
+// whose rows 0..nx-2 form a Dirichlet system cut at the last row.
+struct TileTables
+{
+    int                 P, e;
+    std::vector<double> cc, ends, cp, iden, v, ib;
+};
+TileTables chase_tile_tables(int nx, int R, const std::vector<double>& d, bool start_neu, bool per)
+{
+    const int  ny = (int)d.size(), Ri = R - 1;
+    TileTables t;
+    t.P         = (nx + R - 1) / R;
+    t.e         = nx - t.P * (R - 1);
+    const int P = t.P;
+    t.cc.resize((size_t)2 * Ri * ny);
+    t.ends.resize((size_t)12 * ny);
+    t.cp.resize((size_t)P * ny);
+    t.iden.resize((size_t)P * ny);
+    if (per)
+    {
+        t.v.assign((size_t)P * ny, 0.0);
+        t.ib.resize(ny);
+    }
+    double c[2][16], x[16], e[3][4];
+    for (int j = 0; j < ny; ++j)
+    {
+        const double dj = d[j];
+        for (int typ = 0; typ < 2; ++typ)
+        {
+            c[typ][0] = (typ == 0 && start_neu) ? 1.0 / (dj + 1.0) : 1.0 / dj;
+            for (int r = 1; r < Ri; ++r) c[typ][r] = 1.0 / (dj - c[typ][r - 1]);
+            for (int r = 0; r < Ri; ++r) t.cc[((size_t)typ * Ri + r) * ny + j] = c[typ][r];
+        }
+        for (int k = 0; k < 3; ++k)  // chunk 0, the other long chunks, the short ones
+        {
+            const double* ck = c[k == 0 ? 0 : 1];
+            const int     L  = (k == 0 ? t.e > 0 : k == 1) ? Ri : Ri - 1;
+            for (int which = 0; which < 2; ++which)  // T^-1 e_first, T^-1 e_last
+            {
+                double prev = 0;
+                for (int r = 0; r < L; ++r)
+                {
+                    prev = ((r == (which ? L - 1 : 0) ? 1.0 : 0.0) - prev) * ck[r];
+                    x[r] = prev;
+                }
+                for (int r = L - 2; r >= 0; --r) x[r] -= ck[r] * x[r + 1];
+                e[k][2 * which]     = x[0];
+                e[k][2 * which + 1] = x[L - 1];
+            }
+            for (int w = 0; w < 4; ++w) t.ends[((size_t)k * 4 + w) * ny + j] = e[k][w];
+        }
+        auto   E     = [&](int p) -> const double* { return e[p == 0 ? 0 : p < t.e ? 1 : 2]; };
+        double cprev = 0;
+        for (int p = 0; p < P - 1; ++p)
+        {
+            const double lower = p > 0 ? -E(p)[1] : 0.0;
+            const double inv   = 1.0 / (dj - E(p)[3] - E(p + 1)[0] - lower * cprev);
+            cprev              = -E(p + 1)[2] * inv;
+            t.cp[(size_t)p * ny + j]   = cprev;
+            t.iden[(size_t)p * ny + j] = inv;
+        }
+        if (!per) continue;
+        double D = dj - E(P - 1)[3] - E(0)[0];
+        if (P == 1) D -= E(0)[1] + E(0)[2];
+        else
+        {
+            double yv = 0;
+            for (int p = 0; p < P - 1; ++p)
+            {
+                const double rhs = (p == 0 ? E(0)[1] : 0.0) + (p == P - 2 ? E(P - 1)[2] : 0.0);
+                yv               = (rhs + (p > 0 ? E(p)[1] * yv : 0.0)) * t.iden[(size_t)p * ny + j];
+                t.v[(size_t)p * ny + j] = yv;
+            }
+            for (int p = P - 3; p >= 0; --p)
+                t.v[(size_t)p * ny + j] -= t.cp[(size_t)p * ny + j] * t.v[(size_t)(p + 1) * ny + j];
+            D -= E(P - 1)[1] * t.v[(size_t)(P - 2) * ny + j] + E(0)[2] * t.v[j];
+        }
+        t.ib[j] = 1.0 / D;
+    }
+    return t;
+}
+}  // namespace
+
 template <typename T>
 DevRect<T>::DevRect(int nx_, int ny_, double hx_, double hy_, const int* bc_, int sep_rows, bool with_transform)
     : nx(nx_), ny(ny_), hx(hx_), hy(hy_)
@@ -389,16 +475,37 @@ DevRect<T>::DevRect(int nx_, const std::vector<double>& d, int bc_xneg, int bc_x
 }
 
 // Thomas tables of the nx x ny systems with diagonals d[j] (unit off-diagonals, the x boundary types of bc).
+// sep_rows > 0: the partition tables shared by a batch.
 template <typename T> void DevRect<T>::build_chase_tables(const std::vector<double>& d, int sep_rows)
 {
     const bool xp = bc[XNEG] == BC_PERIODIC && bc[XPOS] == BC_PERIODIC;
     periodic_x    = xp;
+    end_neumann   = !xp && bc[XPOS] == BC_NEUMANN;
+    // the chunked kernels treat only the last wavenumber as singular
+    chunked = !xp && nx % kChunk == 0 && nx >= 2 * kChunk && (!singular || sing_from == ny - 1);
+    tile_R  = tile_rows(nx);
+    tiled   = std::is_same<T, double>::value && tile_R > 0 && sep_rows == 0;
+    if (tiled)
+    {
+        TileTables t = chase_tile_tables(nx, tile_R, d, !xp && bc[XNEG] == BC_NEUMANN, xp);
+        tile_cc      = upload(t.cc);
+        tile_ends    = upload(t.ends);
+        tile_cp      = upload(t.cp);
+        tile_iden    = upload(t.iden);
+        tile_d       = upload(d);
+        if (xp)
+        {
+            tile_v  = upload(t.v);
+            tile_ib = upload(t.ib);
+        }
+        tile_P = t.P;
+        tile_e = t.e;
+    }
+    if (tiled && !singular) return;
     std::vector<double> c;
     chase_table(nx, ny, d, !xp && bc[XNEG] == BC_NEUMANN, !xp && bc[XPOS] == BC_NEUMANN, c);
-    ctab        = upload(convert<T>(c));
-    end_neumann = !xp && bc[XPOS] == BC_NEUMANN;
-    // the chunked kernels treat only the last wavenumber as singular
-    chunked     = !xp && nx % kChunk == 0 && nx >= 2 * kChunk && (!singular || sing_from == ny - 1);
+    ctab = upload(convert<T>(c));
+    if (tiled) return;
     if (chunked)
     {
         std::vector<double> pc, pg, ph, pe;
@@ -423,15 +530,38 @@ template <typename T> void DevRect<T>::build_chase_tables(const std::vector<doub
     }
 }
 
-template <typename T> long long DevRect<T>::chase_scratch_elems(long long batch) const
+template <typename T> long long DevRect<T>::partition_elems(long long batch) const
 {
     if (!chunked) return 0;
     const long long P = nx / kChunk;
     return batch * P * ny * 4;  // chunk end values (2), separator solution (1), separator scan slopes (1)
 }
 
+template <typename T> long long DevRect<T>::chase_scratch_elems(long long batch) const
+{
+    return tiled ? 0 : partition_elems(batch);
+}
+
 template <typename T> void DevRect<T>::chase(T* f, long long batch, T* scr, cudaStream_t s) const
 {
+    if constexpr (std::is_same<T, double>::value)
+        if (tiled)
+        {
+            const ChaseTileTab t{nx, ny, tile_R, tile_P, tile_e, end_neumann ? 1 : 0, periodic_x ? 1 : 0,
+                                 tile_cc.as<double>(), tile_ends.as<double>(), tile_d.as<double>(),
+                                 tile_cp.as<double>(), tile_iden.as<double>(), tile_v.as<double>(),
+                                 tile_ib.as<double>()};
+            const int skip = singular ? ny - sing_from : 0;
+            launch_chase_tile(f, batch, skip, t, s);
+            if (singular)
+            {
+                const long long n = batch * skip;
+                k_chase<T><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(f, nx, ny, batch, ctab.as<T>(), nullptr, nullptr,
+                                                                      periodic_x ? 1 : 0, 1, sing_from, sing_from);
+                FPB_CHECK_LAUNCH();
+            }
+            return;
+        }
     if (!chunked)
     {
         const long long nthreads = batch * ny;
@@ -460,7 +590,7 @@ template <typename T> void DevRect<T>::chase(T* f, long long batch, T* scr, cuda
     if (singular)
     {
         k_chase<T><<<(unsigned)((batch + 127) / 128), 128, 0, s>>>(f, nx, ny, batch, ctab.as<T>(), z1.as<T>(),
-                                                                  z2.as<T>(), 0, 1, 1, ny - 1);
+                                                                  z2.as<T>(), 0, 1, ny - 1, ny - 1);
         FPB_CHECK_LAUNCH();
     }
 }
