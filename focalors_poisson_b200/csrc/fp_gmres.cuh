@@ -79,29 +79,43 @@ __global__ void k_gm_start_basis(double* __restrict__ V, const double* __restric
         V[i] = r[i] * a;
 }
 
-// vin = V_j (the Arnoldi step's input in a fixed buffer); then the projection loop starts at i = 0
-__global__ void k_gm_take(double* __restrict__ vin, const double* __restrict__ V, long long n, GmState* st)
+// vin = V_j (the Arnoldi step's input in a fixed buffer); the projection loop then starts at i = 0
+__global__ void k_gm_take(double* __restrict__ vin, const double* __restrict__ V, long long n, GmState* st,
+                          cudaGraphConditionalHandle mgs)
 {
     const double* v = V + (long long)st->j * n;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         vin[i] = v[i];
-}
-__global__ void k_gm_mgs_begin(GmState* st, cudaGraphConditionalHandle mgs)
-{
-    st->i = 0;
-    cudaGraphSetConditional(mgs, 1u);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        st->i = 0;
+        cudaGraphSetConditional(mgs, 1u);
+    }
 }
 
-// hcol[idx] = a . b with a = V_{st->i} (which = 0) or w (which = 1, idx = j + 1, take the square root)
-__global__ void k_gm_dot(const double* __restrict__ V, const double* __restrict__ w, long long n, const GmState* st,
-                         double* hcol, double* partials, unsigned* ticket, int which)
+// One pass of the modified Gram-Schmidt loop, i = st->i = 0 .. j + 1: w -= hcol[i-1] V_{i-1} (i > 0) and, of the new
+// w, hcol[i] = V_i . w (i <= j) or hcol[j+1] = |w|. One kernel per projection: the subtraction of a projection and
+// the product of the next one read and write w together.
+__global__ void k_gm_project(const double* __restrict__ V, double* __restrict__ w, long long n, GmState* st,
+                             double* hcol, double* partials, unsigned* ticket, cudaGraphConditionalHandle mgs)
 {
     __shared__ double sh[32];
     __shared__ bool   last;
-    const double*     a = which ? w : V + (long long)st->i * n;
+    const int         i = st->i, j = st->j;
+    const double      c = i > 0 ? -hcol[i - 1] : 0.0;
+    const double*     p = V + (long long)(i > 0 ? i - 1 : 0) * n;
+    const double*     a = V + (long long)i * n;
     double            v = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        v += a[i] * w[i];
+    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+    {
+        double x = w[k];
+        if (i > 0)
+        {
+            x += c * p[k];
+            w[k] = x;
+        }
+        v += (i <= j ? a[k] : x) * x;
+    }
     const double s = block_sum(v, sh);
     if (threadIdx.x == 0)
     {
@@ -110,29 +124,15 @@ __global__ void k_gm_dot(const double* __restrict__ V, const double* __restrict_
         last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     }
     __syncthreads();
-    if (last && threadIdx.x == 0)
+    if (!last) return;
+    const double tot = last_block_sum(partials, gridDim.x, sh);
+    if (threadIdx.x == 0)
     {
-        __threadfence();
-        double tot = 0;
-        for (int k = 0; k < (int)gridDim.x; ++k) tot += ((volatile double*)partials)[k];
-        if (which) hcol[st->j + 1] = sqrt(tot);
-        else hcol[st->i] = tot;
+        hcol[i] = i <= j ? tot : sqrt(tot);
         *ticket = 0u;
+        st->i   = i + 1;
+        cudaGraphSetConditional(mgs, i <= j ? 1u : 0u);
     }
-}
-// w -= hcol[i] V_i, then i += 1 and the projection loop goes on while i <= j
-__global__ void k_gm_axpy(double* __restrict__ w, const double* __restrict__ V, long long n, const GmState* st,
-                          const double* hcol)
-{
-    const double  c = -hcol[st->i];
-    const double* v = V + (long long)st->i * n;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        w[i] += c * v[i];
-}
-__global__ void k_gm_mgs_next(GmState* st, cudaGraphConditionalHandle mgs)
-{
-    st->i += 1;
-    cudaGraphSetConditional(mgs, st->i <= st->j ? 1u : 0u);
 }
 
 // V_{j+1} = w / ||w|| (unused after a breakdown)
@@ -299,27 +299,18 @@ cudaGraphExec_t capture_gmres(long long n, int m, double tol, int max_iter, bool
         FPB_CHECK_LAUNCH();
         gm_while(q[1], q[2], inner);
         depth = 3;
-        k_gm_take<<<grid(n, 256, 4096), 256, 0, q[2]>>>(B.vin, B.V, n, B.st);
+        const cudaGraphConditionalHandle mgs = gm_handle(q[2], 0u, false);
+        k_gm_take<<<grid(n, 256, 4096), 256, 0, q[2]>>>(B.vin, B.V, n, B.st, mgs);
         FPB_CHECK_LAUNCH();
         afun(B.vin, B.w, q[2]);
-        const cudaGraphConditionalHandle mgs = gm_handle(q[2], 0u, false);
-        k_gm_mgs_begin<<<1, 1, 0, q[2]>>>(B.st, mgs);
-        FPB_CHECK_LAUNCH();
         gm_while(q[2], q[3], mgs);
         depth = 4;
-        k_gm_dot<<<grid(n, kRedThreads, kRedBlocks), kRedThreads, 0, q[3]>>>(B.V, B.w, n, B.st, B.a.hcol, B.partials,
-                                                                              B.ticket, 0);
-        FPB_CHECK_LAUNCH();
-        k_gm_axpy<<<grid(n, 256, 4096), 256, 0, q[3]>>>(B.w, B.V, n, B.st, B.a.hcol);
-        FPB_CHECK_LAUNCH();
-        k_gm_mgs_next<<<1, 1, 0, q[3]>>>(B.st, mgs);
+        k_gm_project<<<grid(n, kRedThreads, kRedBlocks), kRedThreads, 0, q[3]>>>(B.V, B.w, n, B.st, B.a.hcol, B.partials,
+                                                                                 B.ticket, mgs);
         FPB_CHECK_LAUNCH();
         cudaGraph_t junk = nullptr;
         FPB_CUDA(cudaStreamEndCapture(q[3], &junk));
         depth = 3;
-        k_gm_dot<<<grid(n, kRedThreads, kRedBlocks), kRedThreads, 0, q[2]>>>(B.V, B.w, n, B.st, B.a.hcol, B.partials,
-                                                                              B.ticket, 1);
-        FPB_CHECK_LAUNCH();
         k_gm_next_basis<<<grid(n, 256, 4096), 256, 0, q[2]>>>(B.V, B.w, n, B.st, B.a.hcol);
         FPB_CHECK_LAUNCH();
         k_gm_arnoldi<<<1, 1, 0, q[2]>>>(B.st, B.a, m, inner);
