@@ -1,6 +1,7 @@
 // Batched composite solves (fp_batch.h). Host plan + heterogeneous persistent kernels.
 #include "fp_batch.h"
 #include "fp_chase.cuh"
+#include "fp_dense.h"
 #include "fp_ops.cuh"
 
 #include <cublas_v2.h>
@@ -945,6 +946,7 @@ template <typename T> struct PlanSet  // transform plans by (family, row length)
     std::map<std::pair<int, int>, int>            index;
     std::vector<std::unique_ptr<DevTransform<T>>> tr;
     DevBuf                                        dev;
+    DevBuf                                        dense;  // DenseTab, as dev
     size_t                                        smem       = 0;
     bool                                          stage_only = false;  // plans on the stage engine only
     int get(int kind, int n)
@@ -960,18 +962,21 @@ template <typename T> struct PlanSet  // transform plans by (family, row length)
     void finish()
     {
         std::vector<XformArgs<T>> v;
+        std::vector<DenseTab>     d;
         for (auto& t : tr)
-        {
-            v.push_back(t->args(false));
-            v.push_back(t->args(true));
-        }
-        dev = upload(v);
+            for (bool inv : {false, true})
+            {
+                v.push_back(t->args(inv));
+                d.push_back(t->dense ? t->dense->tab(inv) : DenseTab{});
+            }
+        dev   = upload(v);
+        dense = upload(d);
     }
 };
 
 // A transform work list split by family and engine: one launch per family for its stage-engine plans (the
-// autotuned CTA shape, shared memory of the largest plan) and one per (family, length M) for its
-// register-engine plans (M/16 threads per CTA).
+// autotuned CTA shape, shared memory of the largest plan), one per (family, length M) for its
+// register-engine plans (M/16 threads per CTA) and one per family for its dense plans (fp_dense.cuh).
 struct XList
 {
     struct Part
@@ -980,6 +985,7 @@ struct XList
         int      eng = 0, threads = 0;  // register engine: threads per CTA (stage engine: autotuned)
         size_t   smem = 0;
         int      plan = -1;  // the plan of every run, when they share one (launched with it by value)
+        DenseShape shape;    // dense plans (eng 3): seg holds DenseSeg records, items are row tiles
         Segments seg;
     };
     std::vector<Part> parts;
@@ -988,15 +994,20 @@ struct XList
         parts.clear();
         for (int k : {K_DD, K_ND, K_DN})
         {
-            std::map<int, std::vector<size_t>> groups;  // -1: stage engine, else M of the register engine
+            std::map<int, std::vector<size_t>> groups;  // -1: stage engine, -2: dense, else M of the register engine
             for (size_t i = 0; i < recs.size(); ++i)
                 if (kinds[i] == k)
                 {
                     const FftDesc& d = ps.tr[recs[i].plan]->fd;
-                    groups[d.eng == 1 ? d.M : -1].push_back(i);
+                    groups[d.eng == 1 ? d.M : d.eng == 3 ? -2 : -1].push_back(i);
                 }
             for (auto& g : groups)
             {
+                if (g.first == -2)
+                {
+                    set_dense(k, g.second, recs, ps);
+                    continue;
+                }
                 std::vector<DstSeg>    r;
                 std::vector<long long> c;
                 size_t                 sm   = 0;
@@ -1017,6 +1028,30 @@ struct XList
                 parts.back().seg.set(r, c);
             }
         }
+    }
+    template <typename T>
+    void set_dense(int kind, const std::vector<size_t>& ids, const std::vector<DstSeg>& recs, const PlanSet<T>& ps)
+    {
+        std::vector<DenseLoad> loads;
+        for (size_t i : ids)
+        {
+            const DenseTab t = ps.tr[recs[i].plan]->dense->tab(false);
+            loads.push_back({t.K, t.C, recs[i].rows});
+        }
+        parts.emplace_back();
+        Part& p = parts.back();
+        p.kind  = kind;
+        p.eng   = 3;
+        p.shape = dense_shape(kind, loads);
+        std::vector<DenseSeg>  r;
+        std::vector<long long> c;
+        for (size_t i : ids)
+        {
+            const int n = ps.tr[recs[i].plan]->n;
+            r.push_back({recs[i].in, recs[i].out, 0, recs[i].rows, 1, n, 1, recs[i].plan});
+            c.push_back((recs[i].rows + p.shape.bm - 1) / p.shape.bm);
+        }
+        p.seg.set(r, c);
     }
 };
 
@@ -1075,6 +1110,14 @@ void launch_x(const XList& L, bool inverse, const PlanSet<T>& ps, const BatchTim
     for (auto& part : L.parts)
     {
         const int e = part.eng, th = part.threads, p = part.plan;
+        if (e == 3)
+        {
+            const int omode = std::is_same<TOUT, float>::value ? DENSE_F32 : ACC ? DENSE_ACC : DENSE_F64;
+            dense_launch(part.kind, inverse, part.shape, part.seg.as<DenseSeg>(), part.seg.pre(), part.seg.n,
+                         ps.dense.template as<DenseTab>() + (inverse ? 1 : 0), DenseSeg{}, DenseTab{}, part.seg.total,
+                         std::is_same<TIN, float>::value, omode, s);
+            continue;
+        }
         switch (part.kind)
         {
             case K_DD: launch_x1<T, K_DD, 0, TIN, TOUT, ACC>(part.seg, ps, tm, s, part.smem, e, th, p); break;
@@ -2476,8 +2519,11 @@ template <typename TS> void BatchImpl<TS>::autotune(cudaStream_t s)
     };
     BatchTiming best = tm_;
     float       bt   = 1e30f;
+    bool stage = false;
+    for (auto& part : sg.parts) stage = stage || part.eng == 0;
     for (int th : {128, 192, 256, 384, 512})
     {
+        if (!stage) break;  // nothing the shape would apply to
         int occ = 0;
         FPB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_b_xform<TS, K_DD, 0, TS, TS, false, 0>, th,
                                                                plans_.smem));

@@ -130,6 +130,9 @@ template <typename T> DevBuf upload(const std::vector<T>& v)
     return b;
 }
 
+struct DensePlan;     // fp_dense.h
+struct ChaseTileTab;  // fp_chase_tile.cuh
+
 // Device-resident plan for one transform family at one row length and precision.
 template <typename T> struct DevTransform
 {
@@ -144,6 +147,7 @@ template <typename T> struct DevTransform
     size_t  smem    = 0;
     int     gctas   = 0;
     long long gstride = 0;
+    std::shared_ptr<DensePlan> dense;  // short rows: a product with the matrix (fd.eng = 3, no FFT plan)
 
     // allow_register false: keep the plan on the stage engine (callers that launch plans of several
     // lengths with one CTA shape). allow_global: rows whose FFT buffer exceeds a CTA's shared memory run
@@ -193,6 +197,8 @@ template <typename T> struct DevRect
     // reduced-precision inner solve of iterative refinement. The FP32 transform plan is built on first use.
     void solve_mixed(T* f, long long batch, cudaStream_t s) const;
     mutable std::unique_ptr<DevTransform<float>> tr32;
+    // The one-pass chase's tables for fields of `rows` rows (tiled; rows = nx, or fewer when both are whole chunks).
+    ChaseTileTab tile_tab(int rows) const;
     // Scratch elements the three-pass partition chase would take for `batch` fields (0 where it does not apply).
     long long partition_elems(long long batch) const;
     // Scratch elements the chase needs for `batch` fields.

@@ -1,6 +1,7 @@
 // Device-resident transform and rectangle (PoissonSolver2D) plans.
 #include "fp_chase.cuh"
 #include "fp_chase_tile.cuh"
+#include "fp_dense.h"
 #include "fp_internal.h"
 
 #include <algorithm>
@@ -122,6 +123,12 @@ DevTransform<T>::DevTransform(int kind_, int n_, bool allow_register, bool allow
 {
     if (n < 2) throw Error(1, "row length must be at least 2");
     if (kind == K_PP && (n % 2)) throw Error(1, "periodic transform needs an even length");
+    if (allow_register && n <= dense_limit(kind, std::is_same<T, float>::value))
+    {
+        dense.reset(new DensePlan(kind, n));
+        fd.eng = fd_inv.eng = 3;
+        return;
+    }
     const int L = fft_length(kind, n);
     HostFft   h;
     try
@@ -212,6 +219,12 @@ template <typename TIO>
 void DevTransform<T>::run_io(const TIO* in, TIO* out, long long rows, bool inverse, cudaStream_t s) const
 {
     if (rows > (long long)INT_MAX) throw Error(3, "more than 2^31 rows in one transform call");
+    if (dense)
+    {
+        const bool f32 = std::is_same<TIO, float>::value;
+        dense_rows(*dense, inverse, in, out, rows, f32, f32 ? DENSE_F32 : DENSE_F64, s);
+        return;
+    }
     const DstSeg        a{in, out, (int)rows, 0};
     const int           inv = inverse ? 1 : 0;
     const XformArgs<T>& d   = hargs[inv];
@@ -530,6 +543,14 @@ template <typename T> void DevRect<T>::build_chase_tables(const std::vector<doub
     }
 }
 
+template <typename T> ChaseTileTab DevRect<T>::tile_tab(int rows) const
+{
+    const int P = rows == nx ? tile_P : rows / tile_R;
+    return ChaseTileTab{rows, ny, tile_R, P, rows == nx ? tile_e : P, end_neumann ? 1 : 0, periodic_x ? 1 : 0,
+                        tile_cc.as<double>(), tile_ends.as<double>(), tile_d.as<double>(), tile_cp.as<double>(),
+                        tile_iden.as<double>(), tile_v.as<double>(), tile_ib.as<double>()};
+}
+
 template <typename T> long long DevRect<T>::partition_elems(long long batch) const
 {
     if (!chunked) return 0;
@@ -547,10 +568,7 @@ template <typename T> void DevRect<T>::chase(T* f, long long batch, T* scr, cuda
     if constexpr (std::is_same<T, double>::value)
         if (tiled)
         {
-            const ChaseTileTab t{nx, ny, tile_R, tile_P, tile_e, end_neumann ? 1 : 0, periodic_x ? 1 : 0,
-                                 tile_cc.as<double>(), tile_ends.as<double>(), tile_d.as<double>(),
-                                 tile_cp.as<double>(), tile_iden.as<double>(), tile_v.as<double>(),
-                                 tile_ib.as<double>()};
+            const ChaseTileTab t = tile_tab(nx);
             const int skip = singular ? ny - sing_from : 0;
             launch_chase_tile(f, batch, skip, t, s);
             if (singular)

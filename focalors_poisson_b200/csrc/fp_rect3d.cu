@@ -9,11 +9,13 @@
 //      contiguously, so the 2D chase runs unchanged over ny nz "wavenumbers" with the diagonals
 //      x_diag[k][j] = -2 + (hx/hy)^2 lambda_y[j] + (hx/hz)^2 lambda_z[k] (poisson_solver3d.cpp:57-70)
 //   5. inverse y-transform, transpose back, inverse z-transform.
+// Where the y-transform is a dense product (short ny, fp_dense.cuh) it runs on the middle axis where it lies: steps
+// 2 and the transpose of 5 fall away and the modes stay in the order (j, k).
 // The reference transposes the whole field three times to make each axis contiguous in turn; here only the
 // y axis needs a transpose, because the chase reads its x-lines with one thread per mode (coalesced along
 // the modes).
 #include "../../include/fp_capi.h"
-#include "fp_internal.h"
+#include "fp_dense.h"
 #include "fp_rect3d.h"
 
 #include <cmath>
@@ -87,13 +89,16 @@ DevRect3D::DevRect3D(int nx_, int ny_, int nz_, double hx, double hy, double hz,
     tz.reset(new DevTransform<double>(kz, nz, true, true));
     ty.reset(new DevTransform<double>(ky, ny, true, true));
     const std::vector<double> ly = cal_lambda3(ny, bc[2], bc[3]), lz = cal_lambda3(nz, bc[4], bc[5]);
-    std::vector<double>       d((size_t)ny * nz);
-    for (int k = 0; k < nz; ++k)
-        for (int j = 0; j < ny; ++j)
-            d[(size_t)k * ny + j] = -2.0 + hx * hx / hy / hy * ly[j] + hx * hx / hz / hz * lz[k];
     bool no_dir = true;
     for (int f = 0; f < 6; ++f) no_dir = no_dir && !dir_like(bc[f]);
     const bool xp = bc[0] == BC_PERIODIC && bc[1] == BC_PERIODIC;
+    // in the (i, j, k) layout the singular modes of a periodic x are not the last ones: transposed then
+    in_place = ty->dense && !(no_dir && xp);
+    std::vector<double> d((size_t)ny * nz);
+    for (int k = 0; k < nz; ++k)
+        for (int j = 0; j < ny; ++j)
+            d[in_place ? (size_t)j * nz + k : (size_t)k * ny + j] =
+                -2.0 + hx * hx / hy / hy * ly[j] + hx * hx / hz / hz * lz[k];
     // singular systems without a Dirichlet face (chasing_method3d.cpp:55-90): the last (k, j) pair, or
     // with periodic x every j of the last k
     const int sing_from = xp ? (nz - 1) * ny : nz * ny - 1;
@@ -104,6 +109,17 @@ void DevRect3D::solve(double* f, long long batch, cudaStream_t s) const
 {
     if (batch <= 0) return;
     const long long n = (long long)nx * ny * nz;
+    if (in_place)
+    {
+        const long long need = chase->chase_scratch_elems(batch);
+        if (need) scratch.ensure((size_t)need * sizeof(double));
+        tz->run(f, f, batch * nx * ny, false, s);
+        dense_middle(*ty->dense, false, f, f, batch * nx, nz, s);
+        chase->chase(f, batch, scratch.as<double>(), s);
+        dense_middle(*ty->dense, true, f, f, batch * nx, nz, s);
+        tz->run(f, f, batch * nx * ny, true, s);
+        return;
+    }
     work.ensure((size_t)(batch * n) * sizeof(double));
     double* w = work.as<double>();
     tz->run(f, f, batch * nx * ny, false, s);

@@ -14,6 +14,7 @@ struct DevRect3D
     int                                   nx = 0, ny = 0, nz = 0;
     std::unique_ptr<DevTransform<double>> tz, ty;
     std::unique_ptr<DevRect<double>>      chase;  // nz ny combined modes along x
+    bool                                  in_place = false;  // y-transform on the middle axis, no transposes
     mutable DevBuf                        work, scratch;
 
     // bc: x-, x+, y-, y+, z-, z+ (PDEBoundaryType values; Adjacented faces act as Dirichlet)
