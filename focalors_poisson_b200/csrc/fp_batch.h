@@ -42,7 +42,8 @@ public:
     // precision; steps >= 1: that many inner solves in FP64 iterative refinement (residual of the
     // composite operator in FP64).
     virtual void solve(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s) = 0;
-    // The same launch sequence captured once into a CUDA graph (per field pointers and steps) and replayed.
+    // The same launch sequence captured once into a CUDA graph (per steps) and replayed; other field pointers only
+    // change the records of the work lists that the graph reads.
     virtual void solve_graph(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s) = 0;
     virtual long long graph_kernels() const = 0;  // kernels in the captured graph
     // Iterative refinement until |correction| <= rel_tol |u| over all cells (or the observed contraction
@@ -50,8 +51,8 @@ public:
     // *rel_change the last |correction| / |u|.
     // first: when given, the first inner solve runs on that solver (same problems; e.g. the FP64 solve
     // followed by FP32 corrections).
-    // With max_refine > 1 the whole refinement is one CUDA graph (captured once per field pointers, first
-    // solver and parameters) whose loop over the corrections is a conditional while node: a device kernel
+    // With max_refine > 1 the whole refinement is one CUDA graph (captured once per first solver and
+    // parameters) whose loop over the corrections is a conditional while node: a device kernel
     // applies the stop rule after every correction, so the host waits once, for the result. With
     // max_refine == 1 the loop runs on the host. defer: queue the work and return -1 without waiting;
     // refine_result then gives the outcome once the stream has completed.
@@ -63,9 +64,9 @@ public:
     // One inner solve of already assembled, hx^2-scaled right-hand sides `in` (one pointer per subdomain)
     // into `out` (stored, not accumulated); in and out may alias.
     virtual void solve_assembled(const double* const* in, double* const* out, cudaStream_t s) = 0;
-    // The work lists solve_assembled(in, out, .) uses, built now (outside any stream capture); the
-    // generation counts how often they were rebuilt.
-    virtual void      prepare_assembled(const double* const* in, double* const* out) = 0;
+    // The work lists solve_assembled(in, out, .) uses, built now (outside any stream capture) or refilled in
+    // stream order; the generation counts how often they were rebuilt.
+    virtual void      prepare_assembled(const double* const* in, double* const* out, cudaStream_t s) = 0;
     virtual long long assembled_generation() const = 0;
     // Per-problem |fs - A u| / |fs| (fs: assembled, hx^2-scaled right-hand side); out: host, n_problems.
     virtual void residuals(const double* const* u, const double* const* rhs, const double* const* ghosts,

@@ -93,6 +93,16 @@ void drain(fp_composite* c)
     if (c && c->pipe && c->pipe->pending) FPB_CUDA(cudaStreamSynchronize(c->pipe->out));
 }
 
+// The FP64 spectral solve: its launches as one graph (16 kernels of a few microseconds each on small problems, launched
+// one by one, wait for the host), launched one by one where s is being captured.
+void spectral_solve(BatchBase* b, double* const* f, const double* const* g, cudaStream_t s)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    FPB_CUDA(cudaStreamIsCapturing(s, &cs));
+    if (cs == cudaStreamCaptureStatusNone) b->solve_graph(f, g, 0, s);
+    else b->solve(f, g, 0, s);
+}
+
 // One solve of the given FP_FORM_* on device fields. Returns the batch whose refinement was queued without
 // waiting (defer, spectral refinement forms), else nullptr.
 BatchBase* solve_form(fp_composite* c, double* const* f, const double* const* g, int form, double rel_tol,
@@ -102,7 +112,7 @@ BatchBase* solve_form(fp_composite* c, double* const* f, const double* const* g,
     *change = 0;
     if (form == FP_FORM_F64)
     {
-        if (c->sp64) c->sp64->solve(f, g, 0, s);
+        if (c->sp64) spectral_solve(c->sp64.get(), f, g, s);
         else c->c->solve(f, g, s, gi);
         return nullptr;
     }
@@ -244,7 +254,7 @@ int fp_composite_solve_f64(fp_composite* c, double* const* fields, const double*
     int       rc = guarded([&] {
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         with_device_fields(c, fields, ghosts, flags, s, [&](double* const* f, const double* const* g) {
-            if (c->sp64) c->sp64->solve(f, g, 0, s);  // exact interface solve: nothing to converge
+            if (c->sp64) spectral_solve(c->sp64.get(), f, g, s);  // exact interface solve: nothing to converge
             else c->c->solve(f, g, s, &gi);
         });
         if ((flags & FP_CHECK_CONVERGENCE) && !gi.converged)
@@ -297,7 +307,7 @@ int fp_composite_adjoint_f64(fp_composite* c, double* const* fields, int flags, 
             {
                 c->c->require_nonsingular();
                 c->c->scale_fields(f, false, s);
-                c->sp64->solve(f, nullptr, 0, s);
+                spectral_solve(c->sp64.get(), f, nullptr, s);
                 c->c->scale_fields(f, true, s);
             }
             else

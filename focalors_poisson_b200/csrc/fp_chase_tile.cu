@@ -14,12 +14,12 @@ struct TileFieldIO
     double*   f;
     long long ny;
     __device__ __forceinline__ const double* in(int i, int j) const { return f + i * ny + j; }
-    __device__ __forceinline__ double        rhs(int, int, double v) const { return v; }
     __device__ __forceinline__ double*       out(int i, int j) const { return f + i * ny + j; }
-    __device__ __forceinline__ void          put(double* o, int, int, double x, bool on) const
-    {
-        if (on) *o = x;
-    }
+    __device__ __forceinline__ static constexpr bool store() { return true; }
+    __device__ __forceinline__ void stage() const {}
+    template <int Ri> __device__ __forceinline__ void mods(double (&)[Ri], double&, bool, int, int, int) const {}
+    template <int Ri>
+    __device__ __forceinline__ void take(double (&)[Ri], double, bool, int, int, int, int, bool) const {}
 };
 template <int W, int R>
 __global__ void __launch_bounds__(kTileThreads, 1) k_chase_tile(double* __restrict__ f, int tiles, int skip,

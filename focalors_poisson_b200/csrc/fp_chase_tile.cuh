@@ -7,10 +7,12 @@
 // g = T^-1 e_first, h = T^-1 e_last, and the separators a tridiagonal system of size P whose Thomas factors
 // depend on the wavenumber only and are tabulated:
 //   -g_last B_{p-1} + (d - h_last - g'_first) B_p - h'_first B_{p+1} = f_sep - z_last - z'_first
-// (primes: the next chunk). A pass: the forward elimination of every chunk (its values stay in registers), z_first
-// by a back substitution that stores nothing; the separator system as two affine scans along p (shuffles inside a
-// warp, the warps' compositions through shared memory); then the elimination's values are corrected by B_{p-1} and
-// substituted back from B_p. The Thomas factors c of one chunk serve every sweep and come from shared memory.
+// (primes: the next chunk). With Q_r = (-c_0) .. (-c_{r-1}), a pass is: the forward elimination
+// y_r = (f_r - y_{r-1}) c_r of every chunk, whose values stay in registers, with z_first = sum Q_r y_r beside it; the
+// separator system as two affine scans along p (shuffles inside a warp, the warps' compositions through shared
+// memory); the back substitution x_r = y_r - c_r (x_{r+1} + Q_r B_{p-1}) from x = B_p. The pairs (c_r, Q_r) come from
+// shared memory, one 16-byte read per row and sweep: with the factors read by four sweeps the kernel waited for
+// shared memory (5 x 2048 x 2048 in one launch: 166 us).
 // Periodic x: the last row is a cut, beta = x_{nx-1}. The other separators are solved for beta = 0, the wrapped
 // row gives beta, and their response v to beta = 1 (tabulated) is added.
 // The result equals the sequential Thomas solve (chasing_method_base.cpp:24-52) and, for periodic x, the
@@ -50,7 +52,8 @@ struct ChaseTileTab
     int           R, P, e;     // rows of a long chunk; chunks; the leading ones that are long
     int           end_neu;     // x+ Neumann: the last row's diagonal is d + 1
     int           per;         // periodic x
-    const double* cc;          // [2][R - 1][ny] Thomas factors: first chunk (x- Neumann change), others
+    int           types;       // 2: the first chunk has its own factors (x- Neumann)
+    const double2* cq;         // [types][R - 1][ny] (c_r, Q_r): the other chunks, then the first one's
     const double* ends;        // [3][4][ny] g_first, g_last, h_first, h_last: chunk 0, other long ones, short ones
     const double* d;           // [ny] diagonals
     const double* cp;          // [P][ny] separator Thomas factors; the last row is formed in the kernel
@@ -62,14 +65,14 @@ struct ChaseTileTab
 // Shared memory (doubles) of a CTA of n threads with tiles of W wavenumbers.
 __host__ __device__ __forceinline__ int chase_tile_smem(int n, int W, int R)
 {
-    return 2 * (R - 1) * W + 2 * n + 4 * (n / 32) * W + W;
+    return 4 * (R - 1) * W + 2 * n + 4 * (n / 32) * W + W;
 }
 
 // Inclusive affine scan over the chunks a warp holds (lane stride W), then over the CTA's warps: (a, b) of the
 // thread's own map becomes the value of the composition of every map before and including it, applied to 0.
-// REV: from the last chunk down. ta / tb: the warps' compositions, nw x W each. Contains one barrier.
+// REV: from the last chunk down. tw: the warps' compositions, nw x W. Contains one barrier.
 template <int W, bool REV>
-__device__ __forceinline__ double tile_scan(double a, double b, double* ta, double* tb)
+__device__ __forceinline__ double tile_scan(double a, double b, double2* tw)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, w = lane % W;
     // W = 32: a warp holds one chunk
@@ -85,22 +88,22 @@ __device__ __forceinline__ double tile_scan(double a, double b, double* ta, doub
         }
     }
     if (REV ? lane < W : lane >= 32 - W)
-    {
-        ta[wid * W + w] = a;
-        tb[wid * W + w] = b;
-    }
+        tw[wid * W + w] = make_double2(a, b);
     __syncthreads();
     double y = 0;
-    if (REV)
-        for (int v = nw - 1; v > wid; --v) y = fma(ta[v * W + w], y, tb[v * W + w]);
-    else
-        for (int v = 0; v < wid; ++v) y = fma(ta[v * W + w], y, tb[v * W + w]);
+#pragma unroll 4
+    for (int k = 0; k < (REV ? nw - 1 - wid : wid); ++k)
+    {
+        const double2 m = tw[(REV ? nw - 1 - k : k) * W + w];
+        y               = fma(m.x, y, m.y);
+    }
     return fma(a, y, b);
 }
 
-// One tile. IO: in(i, j) the address of a right-hand side (rows ny apart), rhs(i, j, v) the value from what is
-// there, put(o, i, j, x, on) takes the solution for address o = out(i, j) (called by all
-// threads of a warp together, `on` where there is one). skip: wavenumbers from ny - skip on are left alone. The tile's
+// One tile. IO: in(i, j) the address of a right-hand side (rows ny apart); stage() loads what mods() needs into shared
+// memory (a barrier follows); mods(y, fsep, lng, i0, li, j) turns the thread's values (interior rows i0 + r, separator
+// row i0 + li) into right-hand sides; store() says whether the solution is written, to out(i, j), or handed to
+// take(y, x, lng, p, i0, li, j, on) by all threads of a warp together (interior rows and separator, `on` where valid). skip: wavenumbers from ny - skip on are left alone. The tile's
 // wavenumbers are tile W .. tile W + W - 1; blockDim.x a multiple of 32 of at least P W.
 template <int W, int R, typename IO>
 __device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int skip, const IO& io, double* sm)
@@ -111,14 +114,12 @@ __device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int 
     const int     j0  = tile * W + w;
     const bool    act = p < P && j0 < ny - skip;
     const int     j   = j0 < ny ? j0 : 0;  // idle lanes read column 0 and store nothing
-    double*       cs  = sm;                      // [2][Ri][W]
-    double*       zf  = cs + 2 * Ri * W;         // [n] first interior values; later the separators
-    double*       xs  = zf + n;                  // [n]
-    double*       ta  = xs + n;                  // warps' compositions, forward and backward
-    double*       tb  = ta + (n / 32) * W;
-    double*       ta2 = tb + (n / 32) * W;
-    double*       tb2 = ta2 + (n / 32) * W;
-    double*       sb  = tb2 + (n / 32) * W;      // [W] beta
+    double2*      cs  = reinterpret_cast<double2*>(sm);  // [2][Ri][W]
+    double2*      tw  = cs + 2 * Ri * W;                 // warps' compositions, forward and backward
+    double2*      tw2 = tw + (n / 32) * W;
+    double*       zf  = reinterpret_cast<double*>(tw2 + (n / 32) * W);  // [n] first interior values; later the separators
+    double*       xs  = zf + n;                                         // [n]
+    double*       sb  = xs + n;                                         // [W] beta
     const int     pc  = p < P ? p : P - 1;
     const int     i0  = pc * (R - 1) + min(pc, t.e);
     const bool    lng = pc < t.e;
@@ -129,13 +130,10 @@ __device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int 
 #pragma unroll
     for (int r = 0; r < Ri; ++r, pin += ny) y[r] = r < Ri - 1 || lng ? (double)*pin : 0.0;
     double fsep = (double)*io.in(i0 + li, j);
-#pragma unroll
-    for (int r = 0; r < Ri; ++r)
-        if (r < Ri - 1 || lng) y[r] = io.rhs(i0 + r, j, y[r]);
-    fsep = io.rhs(i0 + li, j, fsep);
-#pragma unroll 4
-    for (int k = tid; k < 2 * Ri * W; k += n)
-        cs[k] = __ldg(t.cc + (long long)(k / W) * ny + min(tile * W + k % W, ny - 1));
+    io.stage();
+#pragma unroll 2
+    for (int k = tid; k < t.types * Ri * W; k += n)
+        cs[k] = __ldg(t.cq + (long long)(k / W) * ny + min(tile * W + k % W, ny - 1));
     // separator row of chunk p (the factors of the last row depend on its being last)
     double        inv = 0, cpv = 0, gl = 0;
     const double* en  = t.ends + (long long)(p == 0 ? 0 : p < t.e ? 1 : 2) * 4 * ny + j;
@@ -155,26 +153,26 @@ __device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int 
     }
     __syncthreads();
 
-    const double* c  = cs + (p == 0 ? 0 : Ri * W) + w;
-    double        zl = 0, z = 0;
+    io.mods(y, fsep, lng, i0, li, j);
+    const double2* c  = cs + (p == 0 && t.types > 1 ? Ri * W : 0) + w;
+    double         zl = 0, z = 0;
 #pragma unroll
     for (int r = 0; r < Ri; ++r)
         if (r < Ri - 1 || lng)
         {
-            zl   = (y[r] - zl) * c[r * W];
-            y[r] = zl;
+            const double2 m = c[r * W];
+            zl              = (y[r] - zl) * m.x;
+            y[r]            = zl;
+            z               = fma(m.y, zl, z);
         }
-#pragma unroll
-    for (int r = Ri - 1; r >= 0; --r)
-        if (r < Ri - 1 || lng) z = fma(-c[r * W], z, y[r]);
     zf[tid] = z;
     __syncthreads();
 
     const bool   sep = p < P - (t.per ? 1 : 0);  // rows of the separator system (the periodic cut is none of them)
     double       rhs = fsep - zl;
     if (p < P - 1) rhs -= zf[tid + W];
-    double x = tile_scan<W, false>(sep ? (p > 0 ? gl * inv : 0.0) : 1.0, sep ? rhs * inv : 0.0, ta, tb);
-    x        = tile_scan<W, true>(sep ? -cpv : 1.0, sep ? x : 0.0, ta2, tb2);
+    double x = tile_scan<W, false>(sep ? (p > 0 ? gl * inv : 0.0) : 1.0, sep ? rhs * inv : 0.0, tw);
+    x        = tile_scan<W, true>(sep ? -cpv : 1.0, sep ? x : 0.0, tw2);
     double bl;
     if (t.per)
     {
@@ -200,22 +198,29 @@ __device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int 
         bl = p > 0 ? xs[tid - W] : 0.0;
     }
 
-    double dl = -bl;
+    if (io.store())
+    {
+        if (act) *io.out(i0 + li, j) = x;
+        auto po = io.out(i0 + Ri - 1, j);
 #pragma unroll
-    for (int r = 0; r < Ri; ++r)
+        for (int r = Ri - 1; r >= 0; --r, po -= ny)
+            if (r < Ri - 1 || lng)
+            {
+                const double2 m = c[r * W];
+                x               = fma(-m.x, fma(m.y, bl, x), y[r]);
+                if (act) *po = x;
+            }
+        return;
+    }
+    const double xsep = x;
+#pragma unroll
+    for (int r = Ri - 1; r >= 0; --r)
         if (r < Ri - 1 || lng)
         {
-            dl *= r ? -c[r * W] : c[0];
-            y[r] += dl;
+            const double2 m = c[r * W];
+            y[r] = x = fma(-m.x, fma(m.y, bl, x), y[r]);
         }
-    io.put(io.out(i0 + li, j), i0 + li, j, x, act);
-    auto po = io.out(i0 + Ri - 1, j);
-#pragma unroll
-    for (int r = Ri - 1; r >= 0; --r, po -= ny)
-    {
-        if (r < Ri - 1 || lng) x = fma(-c[r * W], x, y[r]);
-        io.put(po, i0 + r, j, x, r < Ri - 1 ? act : act && lng);
-    }
+    io.take(y, xsep, lng, p, i0, li, j, act);
 }
 
 // `batch` fields of t.nx x t.ny values back to back, solved in place; wavenumbers from ny - skip on are left alone.

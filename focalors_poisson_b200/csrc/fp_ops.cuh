@@ -394,6 +394,21 @@ __device__ __forceinline__ void dd_acc_prod(double& hi, double& lo, double a, do
     lo += fma(a, b, -p);
 }
 
+// fs - (xm + xp - 2 c + wym ym + wyp yp - 2 r2 c), compensated as above.
+__device__ __forceinline__ double stencil_residual(double fs, double c, double xm, double xp, double ym, double yp,
+                                                   double wym, double wyp, double r2)
+{
+    double hi = xm, lo = 0.0;
+    dd_acc(hi, lo, xp);
+    dd_acc(hi, lo, -2.0 * c);
+    dd_acc_prod(hi, lo, wym, ym);
+    dd_acc_prod(hi, lo, wyp, yp);
+    dd_acc_prod(hi, lo, r2, -2.0 * c);
+    double s, e;
+    two_sum(fs, -hi, s, e);
+    return s + (e - lo);
+}
+
 // fs_t - (A u)_t, compensated as above.
 __device__ __forceinline__ double composite_residual_at(const double* __restrict__ u, double fs, long long t,
                                                         const ResidualArgs& a)
@@ -420,15 +435,7 @@ __device__ __forceinline__ double composite_residual_at(const double* __restrict
     const double xp = (i < nx - 1) ? u[t + ny] : ghost(1, j, c, u[j], wx);
     const double ym = (j > 0) ? u[t - 1] : ghost(2, i, c, u[(long long)i * ny + ny - 1], wym);
     const double yp = (j < ny - 1) ? u[t + 1] : ghost(3, i, c, u[(long long)i * ny], wyp);
-    double       hi = xm, lo = 0.0;
-    dd_acc(hi, lo, xp);
-    dd_acc(hi, lo, -2.0 * c);
-    dd_acc_prod(hi, lo, wym, ym);
-    dd_acc_prod(hi, lo, wyp, yp);
-    dd_acc_prod(hi, lo, a.r2, -2.0 * c);
-    double s, e;
-    two_sum(fs, -hi, s, e);
-    return s + (e - lo);
+    return stencil_residual(fs, c, xm, xp, ym, yp, wym, wyp, a.r2);
 }
 static __global__ void k_composite_residual(double* __restrict__ r, const double* __restrict__ fs,
                                             const double* __restrict__ u, const ResidualArgs a)

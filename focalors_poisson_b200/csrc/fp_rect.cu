@@ -374,8 +374,9 @@ namespace
 // whose rows 0..nx-2 form a Dirichlet system cut at the last row.
 struct TileTables
 {
-    int                 P, e;
-    std::vector<double> cc, ends, cp, iden, v, ib;
+    int                  P, e, types;
+    std::vector<double2> cq;
+    std::vector<double>  ends, cp, iden, v, ib;
 };
 TileTables chase_tile_tables(int nx, int R, const std::vector<double>& d, bool start_neu, bool per)
 {
@@ -384,7 +385,8 @@ TileTables chase_tile_tables(int nx, int R, const std::vector<double>& d, bool s
     t.P         = (nx + R - 1) / R;
     t.e         = nx - t.P * (R - 1);
     const int P = t.P;
-    t.cc.resize((size_t)2 * Ri * ny);
+    t.types     = start_neu ? 2 : 1;
+    t.cq.resize((size_t)t.types * Ri * ny);
     t.ends.resize((size_t)12 * ny);
     t.cp.resize((size_t)P * ny);
     t.iden.resize((size_t)P * ny);
@@ -397,15 +399,20 @@ TileTables chase_tile_tables(int nx, int R, const std::vector<double>& d, bool s
     for (int j = 0; j < ny; ++j)
     {
         const double dj = d[j];
-        for (int typ = 0; typ < 2; ++typ)
+        for (int typ = 0; typ < t.types; ++typ)
         {
-            c[typ][0] = (typ == 0 && start_neu) ? 1.0 / (dj + 1.0) : 1.0 / dj;
+            c[typ][0] = typ == 1 ? 1.0 / (dj + 1.0) : 1.0 / dj;
             for (int r = 1; r < Ri; ++r) c[typ][r] = 1.0 / (dj - c[typ][r - 1]);
-            for (int r = 0; r < Ri; ++r) t.cc[((size_t)typ * Ri + r) * ny + j] = c[typ][r];
+            double q = 1;
+            for (int r = 0; r < Ri; ++r)
+            {
+                t.cq[((size_t)typ * Ri + r) * ny + j] = make_double2(c[typ][r], q);
+                q *= -c[typ][r];
+            }
         }
         for (int k = 0; k < 3; ++k)  // chunk 0, the other long chunks, the short ones
         {
-            const double* ck = c[k == 0 ? 0 : 1];
+            const double* ck = c[k == 0 ? t.types - 1 : 0];
             const int     L  = (k == 0 ? t.e > 0 : k == 1) ? Ri : Ri - 1;
             for (int which = 0; which < 2; ++which)  // T^-1 e_first, T^-1 e_last
             {
@@ -501,7 +508,8 @@ template <typename T> void DevRect<T>::build_chase_tables(const std::vector<doub
     if (tiled)
     {
         TileTables t = chase_tile_tables(nx, tile_R, d, !xp && bc[XNEG] == BC_NEUMANN, xp);
-        tile_cc      = upload(t.cc);
+        tile_cq      = upload(t.cq);
+        tile_types   = t.types;
         tile_ends    = upload(t.ends);
         tile_cp      = upload(t.cp);
         tile_iden    = upload(t.iden);
@@ -547,7 +555,7 @@ template <typename T> ChaseTileTab DevRect<T>::tile_tab(int rows) const
 {
     const int P = rows == nx ? tile_P : rows / tile_R;
     return ChaseTileTab{rows, ny, tile_R, P, rows == nx ? tile_e : P, end_neumann ? 1 : 0, periodic_x ? 1 : 0,
-                        tile_cc.as<double>(), tile_ends.as<double>(), tile_d.as<double>(), tile_cp.as<double>(),
+                        tile_types, tile_cq.as<double2>(), tile_ends.as<double>(), tile_d.as<double>(), tile_cp.as<double>(),
                         tile_iden.as<double>(), tile_v.as<double>(), tile_ib.as<double>()};
 }
 
