@@ -77,14 +77,89 @@ __global__ void k3_plane_add(double* __restrict__ dst, const Plane pd, double a,
     }
 }
 
-// out[t] = f's plane cell t (row-major)
-__global__ void k3_plane_gather(double* __restrict__ out, const double* __restrict__ f, const Plane pf)
+// The children of one box for the Schur apply: all of them in each launch (a step of the GMRES loop is a chain of
+// short kernels: three of them here instead of three per child and a memset).
+struct Kid3
 {
-    const long long n = (long long)pf.np * pf.nq;
+    const double* S;
+    Plane         pp;
+    int           face, cn, off;  // off: the child's part of vec and prod
+};
+struct Kids3
+{
+    Kid3 k[6];
+    int  n, total;
+    int  nx, ny, nz;
+};
+
+// vec = every child's layer of f
+__global__ void k3_gather_kids(double* __restrict__ vec, const double* __restrict__ f, const __grid_constant__ Kids3 K)
+{
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < K.total; t += gridDim.x * blockDim.x)
+    {
+        int c = 0;
+        while (c + 1 < K.n && t >= K.k[c + 1].off) ++c;
+        const Plane& P = K.k[c].pp;
+        const int    q = t - K.k[c].off, a = q / P.nq, b = q - a * P.nq;
+        vec[t]         = f[P.base + a * P.sp + b * P.sq];
+    }
+}
+
+// prod = S vec, child by child; one warp per row, eight loads in flight per lane (the sums keep k_dense_matvec's order).
+// Bound by reading the matrices once: 4 x 2304^2 doubles (170 MB) per step of a 48^3 star.
+__global__ void __launch_bounds__(256) k3_schur_kids(const double* __restrict__ vec, double* __restrict__ prod,
+                                                     const __grid_constant__ Kids3 K)
+{
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= K.total) return;
+    int c = 0;
+    while (c + 1 < K.n && row >= K.k[c + 1].off) ++c;
+    const int     cn = K.k[c].cn;
+    const double* S  = K.k[c].S + (long long)(row - K.k[c].off) * cn;
+    const double* v  = vec + K.k[c].off;
+    double        acc = 0;
+    constexpr int U   = 8;
+    for (int j0 = lane; j0 < cn; j0 += 32 * U)
+    {
+        double a[U], x[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int j = j0 + 32 * u;
+            a[u]        = j < cn ? __ldcs(S + j) : 0.0;
+            x[u]        = j < cn ? v[j] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc += a[u] * x[u];
+    }
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+    if (lane == 0) prod[row] = acc;
+}
+
+// ft = the products on their layers, zero elsewhere (cells of two layers take both, in the children's order)
+__global__ void k3_scatter_kids(double* __restrict__ ft, const double* __restrict__ prod,
+                                const __grid_constant__ Kids3 K)
+{
+    const long long nyz = (long long)K.ny * K.nz, n = K.nx * nyz;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     {
-        const long long p = t / pf.nq, q = t - p * pf.nq;
-        out[t] = f[pf.base + p * pf.sp + q * pf.sq];
+        const long long i = t / nyz;
+        const int       r = (int)(t - i * nyz), j = r / K.nz, l = r - j * K.nz;
+        double    v = 0;
+        for (int c = 0; c < K.n; ++c)
+        {
+            const double* p = prod + K.k[c].off;
+            switch (K.k[c].face)
+            {
+                case 0: if (i == 0) v += p[j * K.nz + l]; break;
+                case 1: if (i == K.nx - 1) v += p[j * K.nz + l]; break;
+                case 2: if (j == 0) v += p[i * K.nz + l]; break;
+                case 3: if (j == K.ny - 1) v += p[i * K.nz + l]; break;
+                case 4: if (l == 0) v += p[i * K.ny + j]; break;
+                default: if (l == K.nz - 1) v += p[i * K.ny + j]; break;
+            }
+        }
+        ft[t] = v;
     }
 }
 
@@ -213,10 +288,10 @@ public:
             const size_t cells = (size_t)box_[d].cells();
             N.V.ensure((size_t)(m_ + 1) * cells * sizeof(double));
             for (DevBuf* b : {&N.w, &N.r, &N.x, &N.ft}) b->ensure(cells * sizeof(double));
-            long long cmax = 0;
-            for (const auto& k : N.kids) cmax = std::max(cmax, k.cn);
-            N.vec.ensure((size_t)cmax * sizeof(double));
-            N.prod.ensure((size_t)cmax * sizeof(double));
+            long long faces = 0;
+            for (const auto& k : N.kids) faces += k.cn;
+            N.vec.ensure((size_t)faces * sizeof(double));
+            N.prod.ensure((size_t)faces * sizeof(double));
             N.hd.ensure((size_t)(m_ + 2) * sizeof(double));
             for (DevBuf* b : {&N.b, &N.vin}) b->ensure(cells * sizeof(double));
             N.arr.ensure((size_t)((m_ + 1) * m_ + 3 * m_ + 1) * sizeof(double));
@@ -362,18 +437,21 @@ private:
         Node3&          N     = node_[d];
         const long long cells = box_[d].cells();
         double*         ft    = N.ft.as<double>();
-        FPB_CUDA(cudaMemsetAsync(ft, 0, cells * sizeof(double), s));
+        Kids3 K{};
+        K.nx = box_[d].nx;
+        K.ny = box_[d].ny;
+        K.nz = box_[d].nz;
         for (const auto& k : N.kids)
         {
-            k3_plane_gather<<<grid3(k.cn, 256), 256, 0, s>>>(N.vec.as<double>(), in, k.pp);
-            FPB_CHECK_LAUNCH();
-            const int warps = 8;
-            k_dense_matvec<<<(unsigned)((k.cn + warps - 1) / warps), warps * 32, 0, s>>>(
-                k.S.as<double>(), (int)k.cn, N.vec.as<double>(), N.prod.as<double>(), 0);
-            FPB_CHECK_LAUNCH();
-            k3_plane_add<<<grid3(k.cn, 256), 256, 0, s>>>(ft, k.pp, 1.0, N.prod.as<double>(), flat_plane(k.pp));
-            FPB_CHECK_LAUNCH();
+            K.k[K.n++] = Kid3{k.S.as<double>(), k.pp, k.face, (int)k.cn, K.total};
+            K.total += (int)k.cn;
         }
+        k3_gather_kids<<<grid3(K.total, 256), 256, 0, s>>>(N.vec.as<double>(), in, K);
+        FPB_CHECK_LAUNCH();
+        k3_schur_kids<<<(unsigned)((K.total + 7) / 8), 256, 0, s>>>(N.vec.as<double>(), N.prod.as<double>(), K);
+        FPB_CHECK_LAUNCH();
+        k3_scatter_kids<<<grid3(cells, 256), 256, 0, s>>>(ft, N.prod.as<double>(), K);
+        FPB_CHECK_LAUNCH();
         rect_[d]->solve(ft, 1, s);
         k_sub<<<grid3(cells, 256), 256, 0, s>>>(out, in, ft, cells);
         FPB_CHECK_LAUNCH();

@@ -131,7 +131,7 @@ template <int KIND, int INV> const void* dense_kernel(int cfg)
     {
         case 0: return (const void*)k_dense<KIND, INV, 1, 2, 4, 2>;
         case 1: return (const void*)k_dense<KIND, INV, 1, 3, 4, 2>;
-        case 2: return (const void*)k_dense<KIND, INV, 1, 4, 4, 2>;
+        case 2: return (const void*)k_dense<KIND, INV, 2, 2, 2, 4>;
         case 3: return (const void*)k_dense<KIND, INV, 1, 5, 4, 2>;
         default: return (const void*)k_dense<KIND, INV, 1, 1, 1, 4>;
     }

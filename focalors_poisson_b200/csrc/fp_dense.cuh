@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
             const DenseTab* __restrict__ tabs, const DenseSeg one, const __grid_constant__ DenseTab tv, int in32,
             int omode, int CS)
 {
-    constexpr int  BM = TM * WM * 8, BN = TN * WN * 8, NT = WM * WN * 32, BK = kDenseBK;
+    constexpr int  BM = TM * WM * 8, BN = TN * WN * 8, NT = WM * WN * 32, NS = kDenseStages, BK = kDenseBK;
     constexpr bool kFold = dense_fold(KIND);
     extern __shared__ __align__(16) double fp_dense_sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -240,36 +240,80 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
             fc += CS;
         }
     };
-    if (iters > 0) fetch(0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < NS - 1; ++i)
+    {
+        if (i < iters) fetch(i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
     // rows into shared memory, folded; zero beyond the rows and columns there are
-    auto fill = [&](auto at) {  // at(r, i): element i of row r
-        auto pair = [&](int r, int t) {
-            double e = 0, o = 0;
-            if (r < rows && t < K) dense_in<KIND, INV>(T, t, [&](int i) -> double { return at(r, i); }, e, o);
-            As[r * lda + t] = e;
-            if (kFold) As[(BM + r) * lda + t] = o;
-        };
-        const int Kp = nk * BK;
-        if (sg.ts == 1)  // lanes along the row
+    // kU pairs per thread are loaded before the first is stored (a load through a generic pointer cannot pass a store to
+    // shared memory by itself)
+    constexpr int kU = 8, NW = NT / 32;
+    const int     Kp = nk * BK;
+    auto          fill_rows = [&](auto* x0) {  // unit stride: lanes along the row
+        const int st = (Kp + 31) / 32, items = BM / NW * st;
+        int       r = warp, t = lane;
+        for (int q0 = 0; q0 < items; q0 += kU)
         {
-            for (int r = warp; r < BM; r += NT / 32)
-#pragma unroll 4
-                for (int t = lane; t < Kp; t += 32) pair(r, t);
-        }
-        else  // lanes across the rows
-        {
-#pragma unroll 4
-            for (int t = tid / BM; t < Kp; t += NT / BM) pair(tid % BM, t);
+            double e[kU], o[kU];
+            int    z[kU];
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+            {
+                const auto* x  = x0 + (long long)r * sg.rs;
+                const bool  in = r < BM && t < Kp;
+                z[u]           = in ? r * lda + t : -1;
+                e[u] = o[u] = 0;
+                if (r < rows && t < K) dense_in<KIND, INV>(T, t, [=](int i) { return (double)x[i]; }, e[u], o[u]);
+                t += 32;
+                if (t >= st * 32)
+                {
+                    t = lane;
+                    r += NW;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+                if (z[u] >= 0)
+                {
+                    As[z[u]] = e[u];
+                    if (kFold) As[BM * lda + z[u]] = o[u];
+                }
         }
     };
+    auto fill_cols = [&](auto* x0) {  // lanes across the rows
+        const int   r = tid % BM;
+        const auto* x = x0 + (long long)r * sg.rs;
+        const int   ts = sg.ts;
+        for (int t0 = tid / BM; t0 < Kp; t0 += kU * (NT / BM))
+        {
+            double e[kU], o[kU];
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+            {
+                const int t = t0 + u * (NT / BM);
+                e[u] = o[u] = 0;
+                if (r < rows && t < K)
+                    dense_in<KIND, INV>(T, t, [=](int i) { return (double)x[(long long)i * ts]; }, e[u], o[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < kU; ++u)
+            {
+                const int t = t0 + u * (NT / BM);
+                if (t >= Kp) continue;
+                As[r * lda + t] = e[u];
+                if (kFold) As[(BM + r) * lda + t] = o[u];
+            }
+        }
+    };
+    if (sg.ts == 1)
     {
-        const float*  f32 = static_cast<const float*>(sg.in) + base;
-        const double* f64 = static_cast<const double*>(sg.in) + base;
-        const long long rs = sg.rs, ts = sg.ts;
-        if (in32) fill([=](int r, int i) { return (double)f32[r * rs + i * ts]; });
-        else fill([=](int r, int i) { return f64[r * rs + i * ts]; });
+        if (in32) fill_rows(static_cast<const float*>(sg.in) + base);
+        else fill_rows(static_cast<const double*>(sg.in) + base);
     }
+    else if (in32) fill_cols(static_cast<const float*>(sg.in) + base);
+    else fill_cols(static_cast<const double*>(sg.in) + base);
     if (CS > 1)  // every CTA of the cluster has read the rows before any of them stores
     {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -287,11 +331,11 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
                 for (int a = 0; a < TM; ++a)
 #pragma unroll
                     for (int b = 0; b < TN; ++b) acc[par][a][b][0] = acc[par][a][b][1] = 0.0;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
         __syncthreads();
-        if (i + 1 < iters) fetch((i + 1) & 1);
+        if (i + NS - 1 < iters) fetch((i + NS - 1) & (NS - 1));
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const double* b0 = Bs + (i & 1) * 2 * BK * (BN + 4) + (lane & 3) * (BN + 4) + wn * TN * 8 + (lane >> 2);
+        const double* b0 = Bs + (i & (NS - 1)) * 2 * BK * (BN + 4) + (lane & 3) * (BN + 4) + wn * TN * 8 + (lane >> 2);
         const double* a0 = As + (wm * TM * 8 + (lane >> 2)) * lda + kc * BK + (lane & 3);
 #pragma unroll
         for (int k = 0; k < BK / 4; ++k)
@@ -320,12 +364,22 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
         const size_t esz = omode == DENSE_F32 ? 4 : 8;
         const bool   vec = sg.ts == 1 && sg.rs % 2 == 0 && (KIND == 0 || T.C % 2 == 0) &&
                          (reinterpret_cast<size_t>(sg.out) + base * esz) % (2 * esz) == 0;
+        const bool   f64 = omode == DENSE_F64 && vec;
 #pragma unroll
         for (int a = 0; a < TM; ++a)
         {
             const int r = wm * TM * 8 + a * 8 + (lane >> 2);
             if (r >= rows) continue;
             const long long ro = base + (long long)r * sg.rs;
+            if (f64)  // the common case apart: its stores are one instruction each
+            {
+                double* const d = static_cast<double*>(sg.out) + ro;
+                auto put  = [=](int q, double v) { d[q] = v; };
+                auto put2 = [=](int q, double u, double v) { *reinterpret_cast<double2*>(d + q) = make_double2(u, v); };
+#pragma unroll
+                for (int b = 0; b < TN; ++b) dense_out<KIND, INV>(T, c0 + b * 8, acc[0][a][b], acc[1][a][b], put, put2);
+                continue;
+            }
             auto put = [&](int q, double v) {
                 const long long z = ro + (long long)q * sg.ts;
                 if (omode == DENSE_F32) static_cast<float*>(sg.out)[z] = (float)v;
@@ -344,14 +398,9 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
                     *reinterpret_cast<float2*>(static_cast<float*>(sg.out) + ro + q) = make_float2((float)u, (float)v);
                     return;
                 }
-                double2* d = reinterpret_cast<double2*>(static_cast<double*>(sg.out) + ro + q);
-                if (omode == DENSE_ACC)
-                {
-                    const double2 w = *d;
-                    u += w.x;
-                    v += w.y;
-                }
-                *d = make_double2(u, v);
+                double2*      d = reinterpret_cast<double2*>(static_cast<double*>(sg.out) + ro + q);  // DENSE_ACC
+                const double2 w = *d;
+                *d              = make_double2(u + w.x, v + w.y);
             };
 #pragma unroll
             for (int b = 0; b < TN; ++b) dense_out<KIND, INV>(T, c0 + b * 8, acc[0][a][b], acc[1][a][b], put, put2);

@@ -106,6 +106,7 @@ __global__ void k_schur_matvec(const double* __restrict__ S, int cn, const T* __
     if (row >= cn) return;
     const double* Sr  = S + (long long)row * cn;
     double        acc = 0.0;
+#pragma unroll 8
     for (int j = lane; j < cn; j += 32) acc += (double)v[j * vstride] * Sr[j];
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if (lane == 0)
@@ -334,6 +335,7 @@ static __global__ void k_dense_matvec(const double* __restrict__ X, int n, const
     if (row >= n) return;
     const double* Xr  = X + (long long)row * n;
     double        acc = 0.0;
+#pragma unroll 8
     for (int j = lane; j < n; j += 32) acc += Xr[j] * g[j];
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     if (lane == 0) y[row] = accumulate ? y[row] + acc : acc;
