@@ -25,18 +25,27 @@ cld root_of_unity(long long num, long long den)  // exp(-2 pi i num / den), exac
     return cld(std::cos(a), std::sin(a));
 }
 
-// Radix sequence for a 7-smooth length (8s first, then 4, 2, 3, 5, 7); empty if not 7-smooth.
-std::vector<int> radices(int m)
+// Radix sequence for a 7-smooth length (empty if it is not). Convolutions: the 8s first, then 4, 2, 3, 5, 7; the last
+// stage's radix is also that of the kernel product, which keeps twice as many values in registers (an 8 there spills
+// at 80 registers: DD 768 FP64 76-79 us against 69 us). Direct transforms: an 8 first, the other 8s last, since the spans
+// between them are then multiples of 8 and a butterfly's shared-memory slots equidistant (slot_stride): NN 576 and PP
+// 576 FP64 34 -> 30 and 55 -> 47 us.
+std::vector<int> radices(int m, bool direct = false)
 {
-    std::vector<int> r;
-    if (m == 1) return r;
-    while (m % 8 == 0) { r.push_back(8); m /= 8; }
-    while (m % 4 == 0) { r.push_back(4); m /= 4; }
-    while (m % 2 == 0) { r.push_back(2); m /= 2; }
-    while (m % 3 == 0) { r.push_back(3); m /= 3; }
-    while (m % 5 == 0) { r.push_back(5); m /= 5; }
-    while (m % 7 == 0) { r.push_back(7); m /= 7; }
-    if (m != 1) r.clear();
+    std::vector<int> r, e;
+    while (m > 1 && m % 8 == 0) { r.push_back(8); m /= 8; }
+    if (direct && r.size() > 1)
+    {
+        e.assign(r.size() - 1, 8);
+        r.resize(1);
+    }
+    while (m > 1 && m % 4 == 0) { r.push_back(4); m /= 4; }
+    while (m > 1 && m % 2 == 0) { r.push_back(2); m /= 2; }
+    while (m > 1 && m % 3 == 0) { r.push_back(3); m /= 3; }
+    while (m > 1 && m % 5 == 0) { r.push_back(5); m /= 5; }
+    while (m > 1 && m % 7 == 0) { r.push_back(7); m /= 7; }
+    if (m != 1) return {};
+    r.insert(r.end(), e.begin(), e.end());
     return r;
 }
 
@@ -108,6 +117,8 @@ void build_stages(FftDesc& d, const std::vector<int>& rad, std::vector<cld>& tw)
         d.st[s].S      = S;
         d.st[s].B      = B;
         d.st[s].tw_off = (int)tw.size();
+        // t / S as a multiplication: exact while t S < 2^32 (t < M / R)
+        d.st[s].inv = (S > 1 && (long long)d.M * d.M / 4 < (1LL << 32)) ? (unsigned)((1ULL << 32) / S + 1) : 0u;
         for (int b = 0; b < S; ++b) tw.push_back(root_of_unity(b, B));
         B = S;
     }
@@ -302,7 +313,7 @@ HostFft plan_fft(int L, size_t elem_bytes, size_t smem_limit, FftWindow fw, FftW
     h.d.L   = L;
     h.d.eng = 0;
     h.d.pad = 3;
-    std::vector<int> rad = radices(L);
+    std::vector<int> rad = radices(L, true);
     if (!rad.empty() || L == 1)
     {
         h.d.M    = L;

@@ -154,7 +154,7 @@ DevTransform<T>::DevTransform(int kind_, int n_, bool allow_register, bool allow
         perm = upload(h.perm);
     }
     std::vector<int4> st(fd.nst);
-    for (int s = 0; s < fd.nst; ++s) st[s] = make_int4(fd.st[s].R, fd.st[s].S, fd.st[s].B, fd.st[s].tw_off);
+    for (int s = 0; s < fd.nst; ++s) st[s] = make_int4(fd.st[s].R, fd.st[s].S, (int)fd.st[s].inv, fd.st[s].tw_off);
     stages        = upload(st);
     KindTables kt = kind_tables(kind, n);
     if (!kt.a.empty())
@@ -522,11 +522,10 @@ template <typename T> void DevRect<T>::build_chase_tables(const std::vector<doub
         tile_P = t.P;
         tile_e = t.e;
     }
-    if (tiled && !singular) return;
+    if (tiled) return;  // the singular wavenumbers' recursion needs no table
     std::vector<double> c;
     chase_table(nx, ny, d, !xp && bc[XNEG] == BC_NEUMANN, !xp && bc[XPOS] == BC_NEUMANN, c);
     ctab = upload(convert<T>(c));
-    if (tiled) return;
     if (chunked)
     {
         std::vector<double> pc, pg, ph, pe;
@@ -582,7 +581,7 @@ template <typename T> void DevRect<T>::chase(T* f, long long batch, T* scr, cuda
             if (singular)
             {
                 const long long n = batch * skip;
-                k_chase<T><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(f, nx, ny, batch, ctab.as<T>(), nullptr, nullptr,
+                k_chase<T><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(f, nx, ny, batch, nullptr, nullptr, nullptr,
                                                                       periodic_x ? 1 : 0, 1, sing_from, sing_from);
                 FPB_CHECK_LAUNCH();
             }
