@@ -62,11 +62,11 @@ __global__ void k_dense_tables(int kind, int inv, int n, int K, int C, int rows,
 }
 }  // namespace
 
-// Where the line lies (us for 4.2 M cells in place, FFT against product, forward / inverse): FP64 DD 256: 72 / 64,
-// 320: 87 / 97; ND 224: about 100 / 94, 256: 95 / 105; NN 96: 55, 60 / 48, 41, 128: 45, 50 / 45, 39, 144: 47, 54 / 62, 56;
-// PP 144: 86, 92 / 69, 60, 192: 62, 64 / 97, 87. Well below it the product wins by more (DD 128: 97 / 39, 64: 176 /
-// 26). FP32 rows keep FP64 arithmetic here, so their line is lower: DD 192: 70 / 49, 256: 45 / 61; ND 192: 90, 106 / 80,
-// 80. 131 k cells: DD 256 13.9 / 8.7, 128 9.2 / 6.0, ND 192 13, 15 / 13, 13.
+// Where the line lies (us for 4.2 M cells in place, FFT against product, forward / inverse): FP64 DD 256: 72 / 63, 320:
+// 83 / 97; ND 224: about 100 / 84, 256: 93, 108 / 105; NN 96: 55, 60 / 48, 41, 128: 43, 48 / 45, 39, 144: 44, 53 / 62,
+// 56; PP 144: 86, 92 / 69, 60, 192: 61, 64 / 97, 87. Well below it the product wins by more (DD 128: 97 / 38, 64: 176 /
+// 27). FP32 rows keep FP64 arithmetic here, so their line is lower: DD 192: 70 / 51, 256: 46 / 61; ND 192: 90, 106 / 75,
+// 75. 131 k cells: DD 256 13.9 / 8.2, 128 9.2 / 5.8, ND 192 13, 15 / 11, 11.
 int dense_limit(int kind, bool f32)
 {
     switch (kind)

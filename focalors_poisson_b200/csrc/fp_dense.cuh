@@ -11,16 +11,17 @@
 // (n + 1, 2 n + 1) several hundred n: dense_limit says where the product stops being the faster one.
 //
 // A CTA takes BM rows whole into shared memory (folded), so that rows may be transformed in place, then runs over
-// column tiles, streaming the table through a two-stage cp.async ring while eight warps accumulate in registers.
+// column tiles, streaming the table through a cp.async ring while eight warps accumulate in registers.
 // A few rows give few CTAs: there a cluster shares a row tile, each CTA loading it and taking every CS-th column
 // tile, with a cluster barrier between the loads and the first store.
 // Rows need not be contiguous: element t of row r sits at r rs + t ts, so the middle axis of a 3D field is
 // transformed where it lies (rs = 1, ts = nz).
 //
 // What bounds it: the FP64 tensor rate (37 TFLOP/s on 148 SMs at 1.965 GHz, the rate of the scalar FP64 pipe; the
-// instruction's gain is 1/8 of the issue slots and operand reads). Measured on 16384 rows of 256 (DD): 64 us, 16.8
-// TFLOP/s, 40 % of the pipe; two waves of CTAs over 296 places and the row loads before a CTA's first product are the
-// rest.
+// instruction's gain is 1/8 of the issue slots and operand reads). Measured on 16384 rows of 256 (DD): 63 us, 17
+// TFLOP/s, 40 % of the pipe. At 4.2 M cells the time is about 15 us, the rows' loads and stores, which overlap little
+// with the products, plus 0.19 us per cell of row length, 60 % of the pipe in the product loop (a third table stage, a
+// deeper ring of half the size and a start of half the CTAs half a tile later all changed less than 3 %).
 #pragma once
 
 #include "fp_common.cuh"
@@ -55,14 +56,17 @@ enum DenseOut
     DENSE_ACC = 2  // FP64 out += result
 };
 
-constexpr int kDenseBK = 16, kDenseStages = 2;
+constexpr int kDenseBK = 16;
+// Table stages in the ring: narrow column tiles multiply for less time than a fetch takes and keep more in flight in
+// the same memory.
+__host__ __device__ constexpr int dense_stages(int bn) { return bn <= 32 ? 4 : bn <= 48 ? 3 : 2; }
 
 __host__ __device__ constexpr bool dense_fold(int kind) { return kind == 0 || kind == 1 || kind == 4; }
 __host__ __device__ __forceinline__ int dense_lda(int K) { return (K + 15) / 16 * 16 + 4; }
 // Shared memory (doubles) of a CTA with row tiles of bm rows and column tiles of bn.
 __host__ __device__ __forceinline__ int dense_smem(bool fold, int K, int bm, int bn)
 {
-    return (fold ? 2 : 1) * bm * dense_lda(K) + kDenseStages * 2 * kDenseBK * (bn + 4);
+    return (fold ? 2 : 1) * bm * dense_lda(K) + dense_stages(bn) * 2 * kDenseBK * (bn + 4);
 }
 
 __device__ __forceinline__ void dense_mma(double (&c)[2], double a, double b)
@@ -185,7 +189,7 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
             const DenseTab* __restrict__ tabs, const DenseSeg one, const __grid_constant__ DenseTab tv, int in32,
             int omode, int CS)
 {
-    constexpr int  BM = TM * WM * 8, BN = TN * WN * 8, NT = WM * WN * 32, NS = kDenseStages, BK = kDenseBK;
+    constexpr int  BM = TM * WM * 8, BN = TN * WN * 8, NT = WM * WN * 32, NS = dense_stages(TN * WN * 8), BK = kDenseBK;
     constexpr bool kFold = dense_fold(KIND);
     extern __shared__ __align__(16) double fp_dense_sm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -333,9 +337,9 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
                     for (int b = 0; b < TN; ++b) acc[par][a][b][0] = acc[par][a][b][1] = 0.0;
         asm volatile("cp.async.wait_group %0;" ::"n"(NS - 2) : "memory");
         __syncthreads();
-        if (i + NS - 1 < iters) fetch((i + NS - 1) & (NS - 1));
+        if (i + NS - 1 < iters) fetch((i + NS - 1) % NS);
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const double* b0 = Bs + (i & (NS - 1)) * 2 * BK * (BN + 4) + (lane & 3) * (BN + 4) + wn * TN * 8 + (lane >> 2);
+        const double* b0 = Bs + (i % NS) * 2 * BK * (BN + 4) + (lane & 3) * (BN + 4) + wn * TN * 8 + (lane >> 2);
         const double* a0 = As + (wm * TM * 8 + (lane >> 2)) * lda + kc * BK + (lane & 3);
 #pragma unroll
         for (int k = 0; k < BK / 4; ++k)
