@@ -1403,8 +1403,8 @@ template <typename T> struct TileList
         for (const Part& p : parts)
             if (p.R == 16)
             {
-                if (p.W == 4 * k) launch1<4 * k, 16>(p, unassembled, store, s);
-                else launch1<2 * k, 16>(p, unassembled, store, s);
+                if (p.W == 4) launch1<4, 16>(p, unassembled, store, s);
+                else if constexpr (k == 2) launch1<8, 16>(p, unassembled, store, s);
             }
             else if (p.R == 8) launch1<8 * k, 8>(p, unassembled, store, s);
             else throw Error(2, "unexpected chunk length");
@@ -1506,7 +1506,7 @@ public:
         if (irhost_) cudaFreeHost(irhost_);
     }
     void solve(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s) override;
-    void solve_graph(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s) override;
+    void solve_graph(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s, bool lazy) override;
     void residuals(const double* const* u, const double* const* rhs, const double* const* ghosts, cudaStream_t s,
                    double* out) override;
     int           n_problems() const override { return (int)prob_.size(); }
@@ -1556,7 +1556,7 @@ private:
     const double* basis_col(int kind, int n, int j);
     bool   build_edge_mv(const std::vector<DstSeg>& segs, const std::vector<int>& ns, Segments& out);
     void   edge_mv(const Segments& l, cudaStream_t s);
-    void   set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s);
+    bool   set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s);
     bool   can_refill(cudaStream_t s);
     ResSeg res_seg(size_t g, double* r, const double* fs, const double* const* u_user);
     void   run(int steps, cudaStream_t s);
@@ -2532,9 +2532,9 @@ template <typename TS> bool BatchImpl<TS>::can_refill(cudaStream_t s)
 
 // Work lists over the caller's fields. Other pointers of the same kind of call only change the records: they are
 // refilled in stream order and the captured graphs stay (a rebuild waits for the device, allocates and captures
-// again: 2.6 of the 3.5 ms of a 5 x 512^2 gradient, whose tensors are new on every call).
+// again: 2.6 of the 3.5 ms of a 5 x 512^2 gradient, whose tensors are new on every call). True: built again.
 template <typename TS>
-void BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s)
+bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s)
 {
     const int nd = (int)dom_.size();
     std::vector<double*>       f(fields, fields + nd);
@@ -2543,7 +2543,7 @@ void BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     if (f == user_ptrs_ && gh == user_ghosts_ && steps == user_steps_)
     {
         user_stream_ = s;
-        return;
+        return false;
     }
     // the ghost pass's list holds the subdomains that have ghosts: the same ones for a refill
     auto ghosted = [&](const std::vector<const double*>& v, int g) {
@@ -2659,12 +2659,13 @@ void BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
             dst_user_in_.refill(di, plans_, s);
             dst_user_out_.refill(dout, plans_, s);
         }
-        return;
+        return false;
     }
     asm_user_.set(as, ac);
     gho_user_.set(gs, gc);
     dst_user_in_.set(di, dst_kinds_, plans_);
     dst_user_out_.set(dout, dst_kinds_, plans_);
+    return true;
 }
 
 template <typename TS> ResSeg BatchImpl<TS>::res_seg(size_t g, double* r, const double* fs, const double* const* u_user)
@@ -2747,11 +2748,21 @@ void BatchImpl<TS>::solve(double* const* fields, const double* const* ghosts, in
 }
 
 template <typename TS> void BatchImpl<TS>::solve_graph(double* const* fields, const double* const* ghosts, int steps,
-                                                       cudaStream_t s)
+                                                       cudaStream_t s, bool lazy)
 {
     if (!fields) throw Error(1, "null field list");
     if (steps < 0 || steps > 64) throw Error(1, "steps must be in [0, 64]");
-    set_user_lists(fields, ghosts, steps, s);
+    const bool built = set_user_lists(fields, ghosts, steps, s);
+    if (lazy)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        FPB_CUDA(cudaStreamIsCapturing(s, &cs));
+        if (cs != cudaStreamCaptureStatusNone || (built && !graph_))
+        {
+            run(steps, s);
+            return;
+        }
+    }
     if (!graph_)
     {
         cudaStream_t cap;

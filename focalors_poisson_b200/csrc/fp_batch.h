@@ -44,7 +44,10 @@ public:
     virtual void solve(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s) = 0;
     // The same launch sequence captured once into a CUDA graph (per steps) and replayed; other field pointers only
     // change the records of the work lists that the graph reads.
-    virtual void solve_graph(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s) = 0;
+    // lazy: the launches are made one by one on a call that has built the lists (a single solve pays for no capture)
+    // and where s is being captured.
+    virtual void solve_graph(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s,
+                             bool lazy = false) = 0;
     virtual long long graph_kernels() const = 0;  // kernels in the captured graph
     // Iterative refinement until |correction| <= rel_tol |u| over all cells (or the observed contraction
     // predicts it after the last correction), at most max_refine inner solves. Returns the steps taken;

@@ -93,14 +93,11 @@ void drain(fp_composite* c)
     if (c && c->pipe && c->pipe->pending) FPB_CUDA(cudaStreamSynchronize(c->pipe->out));
 }
 
-// The FP64 spectral solve: its launches as one graph (16 kernels of a few microseconds each on small problems, launched
-// one by one, wait for the host), launched one by one where s is being captured.
+// The FP64 spectral solve: its launches as one graph from the second call on (16 kernels of a few microseconds each on
+// small problems, launched one by one, wait for the host).
 void spectral_solve(BatchBase* b, double* const* f, const double* const* g, cudaStream_t s)
 {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    FPB_CUDA(cudaStreamIsCapturing(s, &cs));
-    if (cs == cudaStreamCaptureStatusNone) b->solve_graph(f, g, 0, s);
-    else b->solve(f, g, 0, s);
+    b->solve_graph(f, g, 0, s, true);
 }
 
 // One solve of the given FP_FORM_* on device fields. Returns the batch whose refinement was queued without

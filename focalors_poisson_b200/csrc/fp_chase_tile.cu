@@ -45,8 +45,8 @@ template <int W, int R> void launch(double* f, long long batch, int skip, const 
 }  // namespace
 
 // Tile width: 8 wavenumbers (64-byte row pieces) while that keeps a CTA at 512 threads, else 4 (32 bytes, one
-// sector): with 512 threads of 64 registers two tiles share an SM. 2048 x 2048: 27.5 us at 4, 29.7 us at 8; 1000 x
-// 1500: 10.1 us at 4, 11.6 us at 8, 12.8 us at 16.
+// sector): with 512 threads of 64 registers two tiles share an SM. Before the paired factors 2048 x 2048 took
+// 27.5 us at 4, 29.7 us at 8, and 1000 x 1500 10.1 us at 4, 11.6 us at 8, 12.8 us at 16.
 void launch_chase_tile(double* f, long long batch, int skip, const ChaseTileTab& t, cudaStream_t s)
 {
     switch (t.R)

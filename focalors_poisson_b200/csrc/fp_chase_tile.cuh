@@ -12,17 +12,17 @@
 // separator system as two affine scans along p (shuffles inside a warp, the warps' compositions through shared
 // memory); the back substitution x_r = y_r - c_r (x_{r+1} + Q_r B_{p-1}) from x = B_p. The pairs (c_r, Q_r) come from
 // shared memory, one 16-byte read per row and sweep: with the factors read by four sweeps the kernel waited for
-// shared memory (5 x 2048 x 2048 in one launch: 166 us).
+// shared memory (2048 x 2048: 27.5 -> 23.7 us with the pairs).
 // Periodic x: the last row is a cut, beta = x_{nx-1}. The other separators are solved for beta = 0, the wrapped
 // row gives beta, and their response v to beta = 1 (tabulated) is added.
 // The result equals the sequential Thomas solve (chasing_method_base.cpp:24-52) and, for periodic x, the
 // Sherman-Morrison solve (:178-197) up to round-off.
 //
-// What bounds it: one read and one write of the field (L2 or HBM); 2048 x 2048 in 27.5 us, 2.4 TB/s (the three-pass
-// form: 48 us), 256 x 65536 in 79 us, 3.4 TB/s; the load, compute and store phases of the few tiles an SM holds
-// overlap little. At R = 16 the kernel stays at 64 registers, so
-// that an SM holds 1024 threads of tiles, and the dependent chains at 15 steps. Only the last interior row of a
-// chunk is conditional: with a bound on every row the selects took 5/6 of the instructions.
+// What bounds it: one read and one write of the field (L2 or HBM); 2048 x 2048 in 23.7 us, 2.8 TB/s (the three-pass
+// form: 48 us), 256 x 65536 in 81 us, 3.3 TB/s, 1000 x 1500 in 8.6 us (sequential sweep: 764 us); the load, compute
+// and store phases of the few tiles an SM holds overlap little. At R = 16 the kernel stays at 64 registers, so that an
+// SM holds 1024 threads of tiles, and the dependent chains at 15 steps. Only the last interior row of a chunk is
+// conditional: with a bound on every row the selects took 5/6 of the instructions.
 #pragma once
 
 #include "fp_common.cuh"
@@ -35,8 +35,8 @@ constexpr int kTileMaxRows = kTileThreads / 4 * 16;
 
 // Rows of the longer chunks for nx rows, whose chunks of R and R - 1 rows must add up to nx; 0 where none does (nx = 2
 // and 5) or nx is beyond one CTA. 16 above 512 rows; 8 below, where a field gives few tiles and the pass is a chain
-// of latencies (graph replays, 128 x 128 / 384 x 384 / 96 x 11520 periodic: 3.2 / 4.0 / 5.8 us against 4.8 / 4.4 /
-// 8.3 us at R = 16; 2048 x 2048: 34.8 us against 27.5 us).
+// of latencies (graph replays before the paired factors, 128 x 128 / 384 x 384 / 96 x 11520 periodic: 3.2 / 4.0 / 5.8
+// us against 4.8 / 4.4 / 8.3 us at R = 16; 2048 x 2048: 34.8 us against 27.5 us).
 inline int tile_rows(int nx)
 {
     if (nx > kTileMaxRows) return 0;

@@ -3,10 +3,11 @@
 // a fixed memory budget), where a library cudaMalloc would either fail or synchronise the device behind
 // that allocator's back.
 //
-// The partition chase of fp_rect_solve_f64 keeps per-call scratch (chunk end values, the separator
-// solution and the slopes of the separator scan: 4 * batch * (nx/32) * ny doubles) in a buffer the plan grows with
-// cudaMalloc. This variant takes that scratch from one file-scope device array instead, so it calls no
-// allocator at all. Limits and sharing rules are stated next to the array below.
+// The three-pass partition chase that fp_rect_solve_f64 runs on rows beyond 4096 keeps per-call scratch (chunk end
+// values, the separator solution and the slopes of the separator scan: 4 * batch * (nx/32) * ny doubles) in a buffer
+// the plan grows with cudaMalloc. This variant takes that scratch from one file-scope device array instead, so it calls
+// no allocator at all. The limit holds for shorter rows too, whose one-pass chase needs no scratch. Limits and sharing
+// rules are stated next to the array below.
 #include "../../include/fp_capi.h"
 #include "fp_internal.h"
 
