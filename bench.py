@@ -892,12 +892,11 @@ def main():
     torch.cuda.synchronize()
     t_chase = k0.elapsed_time(k1) / reps / 1e3
     ach_chase = bytes_launch / t_chase / 1e9
-    roofline_chase = {"kernel": "k_chase_local + k_chase_reduced + k_chase_correct (2048x2048, FP64, one chase)",
+    roofline_chase = {"kernel": "k_chase_tile (one-pass chase, 2048x2048, FP64)",
                       "bound": "hbm", "achieved": ach_chase, "peak": peak, "unit": "GB/s", "frac": ach_chase / peak,
                       "peak_source": f"{peak_kind} hbm_gbs", "algorithmic_bytes_per_launch": bytes_launch,
                       "avg_launch_ms": t_chase * 1e3,
-                      "traffic_note": "the chase reads and writes the field twice (chunk sweeps, then the "
-                                      "correction): 4*N*8 bytes of DRAM traffic for 2*N*8 algorithmic"}
+                      "traffic_note": "the chase reads and writes the field once, the algorithmic 2*N*8 bytes"}
     del rect, xs
 
     forms = {}
