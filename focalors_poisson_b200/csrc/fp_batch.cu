@@ -1543,6 +1543,17 @@ private:
         DevBuf K;    // root inverse in the 2D basis (problems with both x- and y-edges)
         DevBuf part; // partial sums of the interface's dense products
     };
+    // The work lists over one call's fields and ghosts. steps -1: the records are of no call (a refill failed).
+    struct UserLists
+    {
+        std::vector<double*>       f;
+        std::vector<const double*> ghosts;
+        int                        steps = -1;
+        Segments                   assemble, ghost;  // assembly pass; ghost cells of unassembled fields
+        XList                      in, out;          // one solve in place
+        XList                      iterate, iterate64;  // refinement: inner solutions into the iterate; FP64 plans
+        Segments                   res, add;         // residual; u += r with norms
+    };
 
     void   build_spectral();
     void   build_static_lists();
@@ -1556,10 +1567,14 @@ private:
     const double* basis_col(int kind, int n, int j);
     bool   build_edge_mv(const std::vector<DstSeg>& segs, const std::vector<int>& ns, Segments& out);
     void   edge_mv(const Segments& l, cudaStream_t s);
+    void   build_ir_lists();
     bool   set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s);
     bool   can_refill(cudaStream_t s);
     ResSeg res_seg(size_t g, double* r, const double* fs, const double* const* u_user);
     void   run(int steps, cudaStream_t s);
+    void   assemble(cudaStream_t s);
+    void   residual(cudaStream_t s);
+    void   add_norms(int first, cudaStream_t s);
     void   drop_graphs();
     void   build_ir_graph(double rel_tol, int max_refine, BatchBase* first, const double* const* fi,
                           double* const* fo);
@@ -1572,9 +1587,8 @@ private:
     PlanSet<TS>                               plans_;
     PlanSet<double>                           eplans_;  // FP64 DSTs of edge vectors (length nx of roots)
     // FP32 storage: FP64 plans of the same (family, length) at the same indices as plans_, for the first inner
-    // solve's inverse transform, and the list writing its output into the iterate
+    // solve's inverse transform
     PlanSet<double>                           plans64_;
-    XList                                     dst_out_u64_;
     BatchTiming                               tm64_;
     std::map<std::tuple<int, double, int>, int> tab_index_;
     std::vector<std::unique_ptr<DevRect<double>>> tabs_;  // chase tables (FP64 in both storage precisions)
@@ -1588,7 +1602,6 @@ private:
     TileList<TS>                              tl_leaf_, tl_root_, tl_all_;
     Segments                                  cs_leaf_, cs_root_;  // their column sums
     DevBuf                                    cpart_;
-    Segments                                  gho_user_;           // ghost cells of unassembled fields
     Segments                                  leaf_rows_, leaf_cols_, root_rows_, root_cols_;
     Segments                                  edst_g_, edst_out_;         // FP64 edge DSTs
     Segments                                  edge_mv_g_, edge_mv_o_;     // the same as dense products
@@ -1598,17 +1611,14 @@ private:
     Segments                                  ifyyp_, ifyxp_;              // partial-product blocks
     std::vector<DstSeg>                       dst_W_in_rec_, dst_X_out_rec_;
     std::vector<int>                          dst_kinds_;
-    XList                                     dst_fs_, dst_r_, dst_out_u_, dst_out_r_, dst_user_in_, dst_user_out_;
-    Segments                                  res_, asm_user_;
-    Segments                                  addn_;  // u += r with norms (adaptive refinement)
+    XList                                     dst_fs_, dst_r_, dst_out_r_;  // refinement, between internal buffers
+    bool                                      ir_lists_ = false;            // they and the buffers are there
     DevBuf                                    addp_;
     std::map<std::tuple<int, int, int>, DevBuf> basis_;  // y-basis column tables (family, n, column)
     std::vector<const double*>                ext_in_;     // solve_assembled: last pointer sets and lists
     std::vector<double*>                      ext_out_;
     XList                                     ext_in_list_, ext_out_list_;
-    std::vector<double*>                      user_ptrs_;
-    std::vector<const double*>                user_ghosts_;
-    int                                       user_steps_ = -1;
+    std::unique_ptr<UserLists>                u_;  // of the last call
     cudaStream_t                              user_stream_ = nullptr;
     BatchTiming                               tm_;
     cudaGraphExec_t                           graph_         = nullptr;
@@ -2504,13 +2514,13 @@ void BatchImpl<TS>::inner(const XList& dst_in, const XList& dst_out, bool acc, c
 // solve is ~8e-8 from the answer and one FP32 correction reaches ~3e-13.
 template <typename TS> void BatchImpl<TS>::first_inner(cudaStream_t s)
 {
-    if (std::is_same<TS, float>::value) inner(dst_fs_, dst_out_u64_, false, s, true);
-    else inner(dst_fs_, dst_out_u_, false, s);
+    if (std::is_same<TS, float>::value) inner(dst_fs_, u_->iterate64, false, s, true);
+    else inner(dst_fs_, u_->iterate, false, s);
 }
 
 template <typename TS> void BatchImpl<TS>::build_plans64()
 {
-    if (!std::is_same<TS, float>::value || !plans64_.tr.empty()) return;
+    if (!std::is_same<TS, float>::value || plans64_.dev.get()) return;
     for (auto& D : dom_)
         if (plans64_.get(D.kind, D.d.ny) != D.plan) throw Error(2, "FP64 plan indices differ from the FP32 plans");
     plans64_.finish();
@@ -2530,9 +2540,33 @@ template <typename TS> bool BatchImpl<TS>::can_refill(cudaStream_t s)
     return cs == cudaStreamCaptureStatusNone;
 }
 
+// The refinement's buffers and the lists between them.
+template <typename TS> void BatchImpl<TS>::build_ir_lists()
+{
+    if (ir_lists_) return;
+    fs_.alloc((size_t)cells_ * 8);
+    r_.alloc((size_t)cells_ * 8);
+    std::vector<DstSeg> a = dst_W_in_rec_, b = dst_W_in_rec_, d = dst_X_out_rec_;
+    long long           nb = 0;
+    for (size_t g = 0; g < dom_.size(); ++g)
+    {
+        a[g].in  = fs_.as<double>() + dom_[g].off;
+        b[g].in  = r_.as<double>() + dom_[g].off;
+        d[g].out = r_.as<double>() + dom_[g].off;
+        nb += (dom_[g].d.cells() + kElemCells - 1) / kElemCells;
+    }
+    dst_fs_.set(a, dst_kinds_, plans_);
+    dst_r_.set(b, dst_kinds_, plans_);
+    dst_out_r_.set(d, dst_kinds_, plans_);
+    addp_.alloc((size_t)2 * nb * 8);
+    build_plans64();
+    ir_lists_ = true;
+}
+
 // Work lists over the caller's fields. Other pointers of the same kind of call only change the records: they are
 // refilled in stream order and the captured graphs stay (a rebuild waits for the device, allocates and captures
 // again: 2.6 of the 3.5 ms of a 5 x 512^2 gradient, whose tensors are new on every call). True: built again.
+// A build or refill that fails (out of device memory) leaves no lists behind that a later call would take for its own.
 template <typename TS>
 bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s)
 {
@@ -2540,7 +2574,7 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     std::vector<double*>       f(fields, fields + nd);
     std::vector<const double*> gh;
     if (ghosts) gh.assign(ghosts, ghosts + 4 * nd);
-    if (f == user_ptrs_ && gh == user_ghosts_ && steps == user_steps_)
+    if (u_ && f == u_->f && gh == u_->ghosts && steps == u_->steps)
     {
         user_stream_ = s;
         return false;
@@ -2549,75 +2583,49 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     auto ghosted = [&](const std::vector<const double*>& v, int g) {
         return !v.empty() && (v[4 * g] || v[4 * g + 1] || v[4 * g + 2] || v[4 * g + 3]);
     };
-    bool refill = !user_ptrs_.empty() && steps == user_steps_ && can_refill(s);
-    for (int g = 0; g < nd && refill; ++g) refill = ghosted(gh, g) == ghosted(user_ghosts_, g);
+    bool refill = u_ && steps == u_->steps && can_refill(s);
+    for (int g = 0; g < nd && refill; ++g) refill = ghosted(gh, g) == ghosted(u_->ghosts, g);
+    std::unique_ptr<UserLists> fresh;
     if (!refill)
     {
         drop_graphs();
-        FPB_CUDA(cudaDeviceSynchronize());  // the lists below may still be read by queued work
+        FPB_CUDA(cudaDeviceSynchronize());  // the lists may still be read by queued work
+        fresh.reset(new UserLists());
     }
-    user_ptrs_   = f;
-    user_ghosts_ = gh;
-    user_steps_  = steps;
-    user_stream_ = s;
+    UserLists& L = refill ? *u_ : *fresh;
+    L.steps      = -1;
     const bool ir = steps > 0;
-    if (ir && !fs_.get())
-    {
-        fs_.alloc((size_t)cells_ * 8);
-        r_.alloc((size_t)cells_ * 8);
-        // IR lists between internal buffers
-        std::vector<DstSeg> a = dst_W_in_rec_, b = dst_W_in_rec_;
-        for (size_t g = 0; g < dom_.size(); ++g)
-        {
-            a[g].in = fs_.as<double>() + dom_[g].off;
-            b[g].in = r_.as<double>() + dom_[g].off;
-        }
-        dst_fs_.set(a, dst_kinds_, plans_);
-        dst_r_.set(b, dst_kinds_, plans_);
-        std::vector<DstSeg> d = dst_X_out_rec_;
-        for (size_t g = 0; g < dom_.size(); ++g) d[g].out = r_.as<double>() + dom_[g].off;
-        dst_out_r_.set(d, dst_kinds_, plans_);
-        long long nb = 0;
-        for (size_t g = 0; g < dom_.size(); ++g) nb += (dom_[g].d.cells() + kElemCells - 1) / kElemCells;
-        addp_.alloc((size_t)2 * nb * 8);
-    }
     if (ir)  // the iterate u lives in the caller's fields (their right-hand sides are in fs once assembled)
     {
+        build_ir_lists();
         std::vector<DstSeg> c = dst_X_out_rec_;
         for (int g = 0; g < nd; ++g) c[g].out = f[g];
-        if (refill) dst_out_u_.refill(c, plans_, s);
-        else dst_out_u_.set(c, dst_kinds_, plans_);
-        if (std::is_same<TS, float>::value)
-        {
-            build_plans64();
-            if (refill) dst_out_u64_.refill(c, plans64_, s);
-            else dst_out_u64_.set(c, dst_kinds_, plans64_);
-        }
         const long long        nb = (long long)(addp_.bytes() / 16);
         std::vector<AddSeg>    ad;
-        std::vector<long long> acn;
+        std::vector<ResSeg>    rs;
+        std::vector<long long> blocks;
         long long              b0 = 0;
         for (int g = 0; g < nd; ++g)
         {
-            const long long blocks = (dom_[g].d.cells() + kElemCells - 1) / kElemCells;
+            blocks.push_back((dom_[g].d.cells() + kElemCells - 1) / kElemCells);
             ad.push_back({f[g], r_.as<double>() + dom_[g].off, dom_[g].d.cells(), addp_.as<double>() + b0,
                           addp_.as<double>() + nb + b0});
-            acn.push_back(blocks);
-            b0 += blocks;
+            rs.push_back(res_seg(g, r_.as<double>(), fs_.as<double>(), f.data()));
+            b0 += blocks.back();
         }
-        std::vector<ResSeg>    rs;
-        std::vector<long long> rc;
-        for (int g = 0; g < nd; ++g) rs.push_back(res_seg(g, r_.as<double>(), fs_.as<double>(), f.data()));
-        for (auto& q : rs) rc.push_back((q.a.nx * (long long)q.a.ny + kElemCells - 1) / kElemCells);
         if (refill)
         {
-            addn_.refill(ad, s);
-            res_.refill(rs, s);
+            L.iterate.refill(c, plans_, s);
+            if (std::is_same<TS, float>::value) L.iterate64.refill(c, plans64_, s);
+            L.add.refill(ad, s);
+            L.res.refill(rs, s);
         }
         else
         {
-            addn_.set(ad, acn);
-            res_.set(rs, rc);
+            L.iterate.set(c, dst_kinds_, plans_);
+            if (std::is_same<TS, float>::value) L.iterate64.set(c, dst_kinds_, plans64_);
+            L.add.set(ad, blocks);
+            L.res.set(rs, blocks);
         }
     }
     std::vector<AsmSeg>    as;
@@ -2652,20 +2660,27 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     }
     if (refill)
     {
-        if (ir || !tile_) asm_user_.refill(as, s);
+        if (ir || !tile_) L.assemble.refill(as, s);
         if (!ir)
         {
-            gho_user_.refill(gs, s);
-            dst_user_in_.refill(di, plans_, s);
-            dst_user_out_.refill(dout, plans_, s);
+            L.ghost.refill(gs, s);
+            L.in.refill(di, plans_, s);
+            L.out.refill(dout, plans_, s);
         }
-        return false;
     }
-    asm_user_.set(as, ac);
-    gho_user_.set(gs, gc);
-    dst_user_in_.set(di, dst_kinds_, plans_);
-    dst_user_out_.set(dout, dst_kinds_, plans_);
-    return true;
+    else
+    {
+        L.assemble.set(as, ac);
+        L.ghost.set(gs, gc);
+        L.in.set(di, dst_kinds_, plans_);
+        L.out.set(dout, dst_kinds_, plans_);
+    }
+    L.f          = f;
+    L.ghosts     = gh;
+    L.steps      = steps;
+    user_stream_ = s;
+    if (fresh) u_ = std::move(fresh);
+    return !refill;
 }
 
 template <typename TS> ResSeg BatchImpl<TS>::res_seg(size_t g, double* r, const double* fs, const double* const* u_user)
@@ -2707,32 +2722,49 @@ template <typename TS> ResSeg BatchImpl<TS>::res_seg(size_t g, double* r, const 
     return q;
 }
 
+template <typename TS> void BatchImpl<TS>::assemble(cudaStream_t s)
+{
+    const Segments& l = u_->assemble;
+    k_b_assemble<<<(unsigned)l.total, kElemThreads, 0, s>>>(l.as<AsmSeg>(), l.pre(), l.n);
+    FPB_CHECK_LAUNCH();
+}
+template <typename TS> void BatchImpl<TS>::residual(cudaStream_t s)
+{
+    const Segments& l = u_->res;
+    k_b_residual<<<(unsigned)l.total, kElemThreads, 0, s>>>(l.as<ResSeg>(), l.pre(), l.n);
+    FPB_CHECK_LAUNCH();
+}
+template <typename TS> void BatchImpl<TS>::add_norms(int first, cudaStream_t s)
+{
+    const Segments& l = u_->add;
+    k_b_add_norms<<<(unsigned)l.total, kElemThreads, 0, s>>>(l.as<AddSeg>(), l.pre(), l.n, first);
+    FPB_CHECK_LAUNCH();
+}
+
 template <typename TS> void BatchImpl<TS>::run(int steps, cudaStream_t s)
 {
     if (steps == 0 && tile_)  // the chase applies the hx^2 factor; only ghost values need a pass of their own
     {
-        if (gho_user_.n)
+        const Segments& l = u_->ghost;
+        if (l.n)
         {
-            k_b_ghosts<<<grid_of(gho_user_.total, 256), 256, 0, s>>>(gho_user_.as<GhostSeg>(), gho_user_.pre(),
-                                                                   gho_user_.n);
+            k_b_ghosts<<<grid_of(l.total, 256), 256, 0, s>>>(l.as<GhostSeg>(), l.pre(), l.n);
             FPB_CHECK_LAUNCH();
         }
-        inner(dst_user_in_, dst_user_out_, false, s, false, true);
+        inner(u_->in, u_->out, false, s, false, true);
         return;
     }
-    k_b_assemble<<<(unsigned)asm_user_.total, 256, 0, s>>>(asm_user_.as<AsmSeg>(), asm_user_.pre(), asm_user_.n);
-    FPB_CHECK_LAUNCH();
+    assemble(s);
     if (steps == 0)
     {
-        inner(dst_user_in_, dst_user_out_, false, s);
+        inner(u_->in, u_->out, false, s);
         return;
     }
     first_inner(s);
     for (int k = 1; k < steps; ++k)
     {
-        k_b_residual<<<(unsigned)res_.total, 256, 0, s>>>(res_.as<ResSeg>(), res_.pre(), res_.n);
-        FPB_CHECK_LAUNCH();
-        inner(dst_r_, dst_out_u_, true, s);
+        residual(s);
+        inner(dst_r_, u_->iterate, true, s);
     }
 }
 
@@ -2794,11 +2826,12 @@ template <typename TS> void BatchImpl<TS>::solve_graph(double* const* fields, co
 }
 
 template <typename TS>
-void BatchImpl<TS>::prepare_assembled(const double* const* in, double* const* out, cudaStream_t s)
+void BatchImpl<TS>::prepare_assembled(const double* const* in_ptrs, double* const* out_ptrs,
+                                      cudaStream_t s)
 {
     const int                  nd = (int)dom_.size();
-    std::vector<const double*> vi(in, in + nd);
-    std::vector<double*>       vo(out, out + nd);
+    std::vector<const double*> vi(in_ptrs, in_ptrs + nd);
+    std::vector<double*>       vo(out_ptrs, out_ptrs + nd);
     if (vi == ext_in_ && vo == ext_out_) return;
     std::vector<DstSeg> a = dst_W_in_rec_, b = dst_X_out_rec_;
     for (int g = 0; g < nd; ++g)
@@ -2806,21 +2839,24 @@ void BatchImpl<TS>::prepare_assembled(const double* const* in, double* const* ou
         a[g].in  = vi[g];
         b[g].out = vo[g];
     }
-    if (!ext_in_.empty() && can_refill(s))  // the callers' graphs that hold the lists stay valid: no new generation
+    const bool refill = !ext_in_.empty() && can_refill(s);  // callers' graphs that hold the lists stay valid
+    const bool in = !refill || vi != ext_in_, out = !refill || vo != ext_out_;
+    ext_in_.clear();  // of no call until all is done
+    if (refill)
     {
-        if (vi != ext_in_) ext_in_list_.refill(a, plans_, s);
-        if (vo != ext_out_) ext_out_list_.refill(b, plans_, s);
-        ext_in_  = vi;
-        ext_out_ = vo;
-        return;
+        if (in) ext_in_list_.refill(a, plans_, s);
+        if (out) ext_out_list_.refill(b, plans_, s);
     }
-    FPB_CUDA(cudaDeviceSynchronize());  // the lists below may still be read by queued work
-    user_stream_ = s;
-    ext_in_list_.set(a, dst_kinds_, plans_);
-    ext_out_list_.set(b, dst_kinds_, plans_);
+    else
+    {
+        FPB_CUDA(cudaDeviceSynchronize());  // the lists may still be read by queued work
+        user_stream_ = s;
+        ++ext_gen_;
+        ext_in_list_.set(a, dst_kinds_, plans_);
+        ext_out_list_.set(b, dst_kinds_, plans_);
+    }
     ext_in_  = vi;
     ext_out_ = vo;
-    ++ext_gen_;
 }
 
 template <typename TS>
@@ -2846,8 +2882,7 @@ void BatchImpl<TS>::build_ir_graph(double rel_tol, int max_refine, BatchBase* fi
         FPB_CUDA(cudaStreamCreateWithFlags(&cb, cudaStreamNonBlocking));
         FPB_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
         in_cap = true;
-        k_b_assemble<<<(unsigned)asm_user_.total, 256, 0, cap>>>(asm_user_.as<AsmSeg>(), asm_user_.pre(), asm_user_.n);
-        FPB_CHECK_LAUNCH();
+        assemble(cap);
         if (first) first->solve_assembled(fi, fo, cap);
         else first_inner(cap);
         k_ir_init<<<1, 1, 0, cap>>>(irst_.as<IrState>());
@@ -2871,11 +2906,9 @@ void BatchImpl<TS>::build_ir_graph(double rel_tol, int max_refine, BatchBase* fi
         FPB_CUDA(cudaStreamBeginCaptureToGraph(cb, np.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                                cudaStreamCaptureModeThreadLocal));
         in_body = true;
-        k_b_residual<<<(unsigned)res_.total, 256, 0, cb>>>(res_.as<ResSeg>(), res_.pre(), res_.n);
-        FPB_CHECK_LAUNCH();
+        residual(cb);
         inner(dst_r_, dst_out_r_, false, cb);
-        k_b_add_norms<<<(unsigned)addn_.total, 256, 0, cb>>>(addn_.as<AddSeg>(), addn_.pre(), addn_.n, 0);
-        FPB_CHECK_LAUNCH();
+        add_norms(0, cb);
         const long long nb = (long long)(addp_.bytes() / 16);
         k_ir_check<<<1, 256, 0, cb>>>(addp_.as<double>(), nb, irst_.as<IrState>(), rel_tol, max_refine, loop);
         FPB_CHECK_LAUNCH();
@@ -2958,7 +2991,7 @@ int BatchImpl<TS>::refine(double* const* fields, const double* const* ghosts, do
         for (int g = 0; g < nd; ++g)
         {
             fi[g] = fs_.as<double>() + dom_[g].off;
-            fo[g] = user_ptrs_[g];
+            fo[g] = u_->f[g];
         }
         if (first) first->prepare_assembled(fi.data(), fo.data(), s);
         if (!irst_.get())
@@ -2988,8 +3021,7 @@ int BatchImpl<TS>::refine(double* const* fields, const double* const* ghosts, do
         return ir_outcome(rel_change, runs);
     }
     // max_refine == 1: one inner solve into r, then u = r through the add pass, whose norms check the values
-    k_b_assemble<<<(unsigned)asm_user_.total, 256, 0, s>>>(asm_user_.as<AsmSeg>(), asm_user_.pre(), asm_user_.n);
-    FPB_CHECK_LAUNCH();
+    assemble(s);
     if (first)
     {
         std::vector<const double*> fi(dom_.size());
@@ -3003,8 +3035,7 @@ int BatchImpl<TS>::refine(double* const* fields, const double* const* ghosts, do
     }
     else
         inner(dst_fs_, dst_out_r_, false, s);
-    k_b_add_norms<<<(unsigned)addn_.total, 256, 0, s>>>(addn_.as<AddSeg>(), addn_.pre(), addn_.n, 1);
-    FPB_CHECK_LAUNCH();
+    add_norms(1, s);
     const long long     nb = (long long)(addp_.bytes() / 16);
     std::vector<double> hp((size_t)2 * nb);
     FPB_CUDA(cudaMemcpyAsync(hp.data(), addp_.get(), hp.size() * 8, cudaMemcpyDeviceToHost, s));

@@ -56,8 +56,11 @@ template <typename F> int guarded(F&& f)
     {                                                                                                    \
         cudaError_t e_ = (call);                                                                         \
         if (e_ != cudaSuccess)                                                                           \
+        {                                                                                                \
+            (void)cudaGetLastError(); /* reported here, not again by the next launch's check */          \
             throw ::fpb::Error(e_ == cudaErrorMemoryAllocation ? 6 : 2,                                  \
                                std::string(#call) + ": " + cudaGetErrorString(e_));                      \
+        }                                                                                                \
     } while (0)
 
 // Every kernel launch is followed by FPB_CHECK_LAUNCH(), which also counts it (fp_launch_count()).
