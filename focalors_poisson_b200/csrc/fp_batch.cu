@@ -1569,7 +1569,6 @@ private:
     void   edge_mv(const Segments& l, cudaStream_t s);
     void   build_ir_lists();
     bool   set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s);
-    bool   can_refill(cudaStream_t s);
     ResSeg res_seg(size_t g, double* r, const double* fs, const double* const* u_user);
     void   run(int steps, cudaStream_t s);
     void   assemble(cudaStream_t s);
@@ -1619,7 +1618,6 @@ private:
     std::vector<double*>                      ext_out_;
     XList                                     ext_in_list_, ext_out_list_;
     std::unique_ptr<UserLists>                u_;  // of the last call
-    cudaStream_t                              user_stream_ = nullptr;
     BatchTiming                               tm_;
     cudaGraphExec_t                           graph_         = nullptr;
     long long                                 graph_kernels_ = 0;
@@ -2529,17 +2527,6 @@ template <typename TS> void BatchImpl<TS>::build_plans64()
     tm64_.dst_blocks_per_sm = 1 << 20;  // one CTA per work item
 }
 
-// Whether the work lists of the last call may be refilled in stream order for a call on s with other pointers: on the
-// stream of that call nothing else orders this call after it, so any other stream waits for the device as a rebuild
-// does; a capture would record the refill's copy instead of making it.
-template <typename TS> bool BatchImpl<TS>::can_refill(cudaStream_t s)
-{
-    if (s != user_stream_ || s == cudaStreamPerThread) return false;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    FPB_CUDA(cudaStreamIsCapturing(s, &cs));
-    return cs == cudaStreamCaptureStatusNone;
-}
-
 // The refinement's buffers and the lists between them.
 template <typename TS> void BatchImpl<TS>::build_ir_lists()
 {
@@ -2564,7 +2551,7 @@ template <typename TS> void BatchImpl<TS>::build_ir_lists()
 }
 
 // Work lists over the caller's fields. Other pointers of the same kind of call only change the records: they are
-// refilled in stream order and the captured graphs stay (a rebuild waits for the device, allocates and captures
+// refilled in the order of the calls (`order`) and the captured graphs stay (a rebuild waits for the device, allocates and captures
 // again: 2.6 of the 3.5 ms of a 5 x 512^2 gradient, whose tensors are new on every call). True: built again.
 // A build or refill that fails (out of device memory) leaves no lists behind that a later call would take for its own.
 template <typename TS>
@@ -2574,16 +2561,12 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     std::vector<double*>       f(fields, fields + nd);
     std::vector<const double*> gh;
     if (ghosts) gh.assign(ghosts, ghosts + 4 * nd);
-    if (u_ && f == u_->f && gh == u_->ghosts && steps == u_->steps)
-    {
-        user_stream_ = s;
-        return false;
-    }
+    if (u_ && f == u_->f && gh == u_->ghosts && steps == u_->steps) return false;
     // the ghost pass's list holds the subdomains that have ghosts: the same ones for a refill
     auto ghosted = [&](const std::vector<const double*>& v, int g) {
         return !v.empty() && (v[4 * g] || v[4 * g + 1] || v[4 * g + 2] || v[4 * g + 3]);
     };
-    bool refill = u_ && steps == u_->steps && can_refill(s);
+    bool refill = u_ && steps == u_->steps && !is_capturing(s);  // a capture would only record the copies
     for (int g = 0; g < nd && refill; ++g) refill = ghosted(gh, g) == ghosted(u_->ghosts, g);
     std::unique_ptr<UserLists> fresh;
     if (!refill)
@@ -2593,7 +2576,7 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
         fresh.reset(new UserLists());
     }
     UserLists& L = refill ? *u_ : *fresh;
-    L.steps      = -1;
+    L.steps       = -1;
     const bool ir = steps > 0;
     if (ir)  // the iterate u lives in the caller's fields (their right-hand sides are in fs once assembled)
     {
@@ -2675,10 +2658,9 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
         L.in.set(di, dst_kinds_, plans_);
         L.out.set(dout, dst_kinds_, plans_);
     }
-    L.f          = f;
-    L.ghosts     = gh;
-    L.steps      = steps;
-    user_stream_ = s;
+    L.f      = f;
+    L.ghosts = gh;
+    L.steps  = steps;
     if (fresh) u_ = std::move(fresh);
     return !refill;
 }
@@ -2775,6 +2757,7 @@ void BatchImpl<TS>::solve(double* const* fields, const double* const* ghosts, in
     for (int g = 0; g < (int)dom_.size(); ++g)
         if (!fields[g]) throw Error(1, "null field pointer");
     if (steps < 0 || steps > 64) throw Error(1, "steps must be in [0, 64]");
+    const StreamOrder::Call call(&order, s);
     set_user_lists(fields, ghosts, steps, s);
     run(steps, s);
 }
@@ -2784,16 +2767,12 @@ template <typename TS> void BatchImpl<TS>::solve_graph(double* const* fields, co
 {
     if (!fields) throw Error(1, "null field list");
     if (steps < 0 || steps > 64) throw Error(1, "steps must be in [0, 64]");
-    const bool built = set_user_lists(fields, ghosts, steps, s);
-    if (lazy)
+    const StreamOrder::Call call(&order, s);
+    const bool              built = set_user_lists(fields, ghosts, steps, s);
+    if (lazy && (built || is_capturing(s)))
     {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        FPB_CUDA(cudaStreamIsCapturing(s, &cs));
-        if (cs != cudaStreamCaptureStatusNone || (built && !graph_))
-        {
-            run(steps, s);
-            return;
-        }
+        run(steps, s);
+        return;
     }
     if (!graph_)
     {
@@ -2839,7 +2818,7 @@ void BatchImpl<TS>::prepare_assembled(const double* const* in_ptrs, double* cons
         a[g].in  = vi[g];
         b[g].out = vo[g];
     }
-    const bool refill = !ext_in_.empty() && can_refill(s);  // callers' graphs that hold the lists stay valid
+    const bool refill = !ext_in_.empty() && !is_capturing(s);  // callers' graphs that hold the lists stay valid
     const bool in = !refill || vi != ext_in_, out = !refill || vo != ext_out_;
     ext_in_.clear();  // of no call until all is done
     if (refill)
@@ -2850,7 +2829,6 @@ void BatchImpl<TS>::prepare_assembled(const double* const* in_ptrs, double* cons
     else
     {
         FPB_CUDA(cudaDeviceSynchronize());  // the lists may still be read by queued work
-        user_stream_ = s;
         ++ext_gen_;
         ext_in_list_.set(a, dst_kinds_, plans_);
         ext_out_list_.set(b, dst_kinds_, plans_);
@@ -2982,6 +2960,7 @@ int BatchImpl<TS>::refine(double* const* fields, const double* const* ghosts, do
 {
     if (!fields) throw Error(1, "null field list");
     if (!(rel_tol > 0) || max_refine < 1) throw Error(1, "rel_tol must be > 0 and max_refine >= 1");
+    const StreamOrder::Call call(&order, s), first_call(first && first != this ? &first->order : nullptr, s);
     set_user_lists(fields, ghosts, 1, s);
     if (max_refine > 1)
     {

@@ -43,7 +43,7 @@ public:
     // composite operator in FP64).
     virtual void solve(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s) = 0;
     // The same launch sequence captured once into a CUDA graph (per steps) and replayed; other field pointers only
-    // change the records of the work lists that the graph reads.
+    // change the records of the work lists that the graph reads. Calls on several streams run one after the other.
     // lazy: the launches are made one by one on a call that has built the lists (a single solve pays for no capture)
     // and where s is being captured.
     virtual void solve_graph(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s,
@@ -79,6 +79,7 @@ public:
     virtual const Domain& domain(int g) const = 0;
     virtual BatchTiming   timing() const      = 0;
     virtual void          autotune(cudaStream_t s) = 0;
+    StreamOrder           order;  // of the calls that use the work buffers and lists
 };
 
 // precision: 0 = FP64 storage and arithmetic, 1 = FP32 storage and arithmetic in the inner solves.

@@ -133,6 +133,52 @@ template <typename T> DevBuf upload(const std::vector<T>& v)
     return b;
 }
 
+inline bool is_capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    FPB_CUDA(cudaStreamIsCapturing(s, &cs));
+    return cs != cudaStreamCaptureStatusNone;
+}
+
+// Queues the calls on one object's buffers one after the other, whatever streams they come on: each waits for an event
+// recorded at the end of the one before (an equal stream handle proves no order, it may have been destroyed with work
+// queued and given out again). A call being captured is left out; its graph's launches are the caller's to order.
+class StreamOrder
+{
+public:
+    StreamOrder() = default;
+    ~StreamOrder()
+    {
+        if (e_) cudaEventDestroy(e_);
+    }
+    StreamOrder(const StreamOrder&)            = delete;
+    StreamOrder& operator=(const StreamOrder&) = delete;
+    // One call on `s`; a null object orders nothing.
+    class Call
+    {
+    public:
+        Call(StreamOrder* o, cudaStream_t s) : o_(o && !is_capturing(s) ? o : nullptr), s_(s)
+        {
+            if (!o_) return;
+            if (!o_->e_) FPB_CUDA(cudaEventCreateWithFlags(&o_->e_, cudaEventDisableTiming));
+            else FPB_CUDA(cudaStreamWaitEvent(s_, o_->e_, 0));
+        }
+        ~Call()
+        {
+            if (o_ && cudaEventRecord(o_->e_, s_) != cudaSuccess) (void)cudaGetLastError();
+        }
+        Call(const Call&)            = delete;
+        Call& operator=(const Call&) = delete;
+
+    private:
+        StreamOrder* o_;
+        cudaStream_t s_;
+    };
+
+private:
+    cudaEvent_t e_ = nullptr;
+};
+
 struct DensePlan;     // fp_dense.h
 struct ChaseTileTab;  // fp_chase_tile.cuh
 

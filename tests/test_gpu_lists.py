@@ -46,3 +46,66 @@ def test_no_lists_left_by_a_call_out_of_memory(retry):
     one.solve(got, steps=2)
     torch.cuda.synchronize()
     assert _same(torch, got, want)
+
+
+def test_calls_queued_on_one_stream_and_on_two():
+    """Calls on other fields follow each other without a wait of the host: the lists of a solve still running must not
+    change. On two streams ordered by nothing else the solver orders its own calls."""
+    torch = torch_cuda()
+    g = W.cross(512, neumann_tips=True)
+    one = capi.Composite(g, m=20, tol=1e-12, max_iter=100)
+    batch = capi.Batch([g, W.cross(256)], precision="f32")
+    sets = [_rhs(torch, g, k) for k in range(6)]
+    more = [_rhs(torch, g, k) + _rhs(torch, W.cross(256), k) for k in range(6)]
+    fresh = capi.Composite(g, m=20, tol=1e-12, max_iter=100)
+    calls = [(fresh.solve, one.solve), (fresh.adjoint, one.adjoint)] * 3
+    want = [_solved(torch, c[0], f) for c, f in zip(calls, sets)]
+    same = capi.Batch([g, W.cross(256)], precision="f32")
+    bwant = [_solved(torch, lambda x: same.solve(x, steps=2), f) for f in more]
+    for streams in (1, 2):
+        lanes = [torch.cuda.Stream() for _ in range(streams)]
+        got, bgot = [[x.clone() for x in f] for f in sets], [[x.clone() for x in f] for f in more]
+        torch.cuda.synchronize()
+        for k in range(6):
+            with torch.cuda.stream(lanes[k % streams]):
+                calls[k][1](got[k])
+                batch.solve(bgot[k], steps=2, graph=True)
+        torch.cuda.synchronize()
+        for k in range(6):
+            assert _same(torch, got[k], want[k]) and _same(torch, bgot[k], bwant[k]), (streams, k)
+
+
+def test_stream_handle_given_out_again():
+    """A stream is destroyed with a solve still queued on it, and the next stream may get its handle: a solve of other
+    fields there must leave the queued one its lists."""
+    import ctypes
+
+    torch = torch_cuda()
+    g = W.cross(64)
+    one = capi.Composite(g, m=20, tol=1e-12, max_iter=100)
+    a, b = _rhs(torch, g, 1), _rhs(torch, g, 2)
+    rhs = [x.clone() for x in a]
+    fresh = capi.Composite(g, m=20, tol=1e-12, max_iter=100)
+    want_a, want_b = _solved(torch, fresh.solve, a), _solved(torch, fresh.solve, b)
+    rt = torch.cuda.cudart()
+
+    def stream():
+        h = ctypes.c_void_p()
+        assert int(rt.cudaStreamCreate(ctypes.addressof(h))) == 0
+        return h.value
+
+    first = stream()
+    with torch.cuda.stream(torch.cuda.ExternalStream(first)):
+        one.solve(a)
+        one.solve(a)
+        for x, y in zip(a, rhs):
+            x.copy_(y)
+        torch.cuda._sleep(400_000_000)  # 0.2 s
+        one.solve(a)
+    assert int(rt.cudaStreamDestroy(first)) == 0
+    second = stream()
+    with torch.cuda.stream(torch.cuda.ExternalStream(second)):
+        one.solve(b)
+    torch.cuda.synchronize()
+    assert _same(torch, a, want_a) and _same(torch, b, want_b), second == first
+    assert int(rt.cudaStreamDestroy(second)) == 0
