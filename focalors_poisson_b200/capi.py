@@ -628,7 +628,8 @@ class Batch:
 
     def solve(self, fields, ghosts=None, steps=0, graph=False, sync=False):
         """In place. steps == 0: one solve in the storage precision; steps >= 1: FP64 iterative refinement
-        with that many inner solves. graph: capture once, replay afterwards (same tensors and steps)."""
+        with that many inner solves. graph: capture once per number of steps, replay afterwards; other tensors
+        only change the work lists that the graph reads."""
         flags = FP_DEVICE | (FP_BATCH_GRAPH if graph else 0) | (FP_SYNC if sync else 0)
         check(lib().fp_batch_solve(self.h, self._ptrs(fields), self._ghosts(ghosts), flags, _stream(), int(steps)))
 

@@ -9,8 +9,10 @@
 #include <cusolverDn.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <map>
+#include <memory>
 #include <numeric>
 #include <type_traits>
 
@@ -1553,6 +1555,8 @@ private:
         XList                      in, out;          // one solve in place
         XList                      iterate, iterate64;  // refinement: inner solutions into the iterate; FP64 plans
         Segments                   res, add;         // residual; u += r with norms
+        // captured graphs of the caller's that read the lists; counted by objects those graphs own
+        std::shared_ptr<std::atomic<int>> graphs = std::make_shared<std::atomic<int>>(0);
     };
 
     void   build_spectral();
@@ -1568,6 +1572,7 @@ private:
     bool   build_edge_mv(const std::vector<DstSeg>& segs, const std::vector<int>& ns, Segments& out);
     void   edge_mv(const Segments& l, cudaStream_t s);
     void   build_ir_lists();
+    void   note_capture(cudaStream_t s);
     bool   set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s);
     ResSeg res_seg(size_t g, double* r, const double* fs, const double* const* u_user);
     void   run(int steps, cudaStream_t s);
@@ -1618,6 +1623,7 @@ private:
     std::vector<double*>                      ext_out_;
     XList                                     ext_in_list_, ext_out_list_;
     std::unique_ptr<UserLists>                u_;  // of the last call
+    std::vector<std::unique_ptr<UserLists>>   captured_;  // of earlier calls, still read by graphs of the caller's
     BatchTiming                               tm_;
     cudaGraphExec_t                           graph_         = nullptr;
     long long                                 graph_kernels_ = 0;
@@ -2550,6 +2556,28 @@ template <typename TS> void BatchImpl<TS>::build_ir_lists()
     ir_lists_ = true;
 }
 
+// The call on s is being captured: the graph owns a reference to the lists that it will read, so that they are neither
+// refilled nor freed while it or an executable graph made from it exists.
+template <typename TS> void BatchImpl<TS>::note_capture(cudaStream_t s)
+{
+    using Count = std::shared_ptr<std::atomic<int>>;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    cudaGraph_t             g  = nullptr;
+    FPB_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, nullptr, nullptr));
+    std::unique_ptr<Count> held(new Count(u_->graphs));
+    cudaUserObject_t       o   = nullptr;
+    const cudaHostFn_t     end = [](void* p) {
+        Count* c = static_cast<Count*>(p);
+        --**c;
+        delete c;
+    };
+    FPB_CUDA(cudaUserObjectCreate(&o, held.get(), end, 1, cudaUserObjectNoDestructorSync));
+    ++**held.release();  // `end` undoes it
+    const cudaError_t e = cudaGraphRetainUserObject(g, o, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) cudaUserObjectRelease(o, 1);
+    FPB_CUDA(e);
+}
+
 // Work lists over the caller's fields. Other pointers of the same kind of call only change the records: they are
 // refilled in the order of the calls (`order`) and the captured graphs stay (a rebuild waits for the device, allocates and captures
 // again: 2.6 of the 3.5 ms of a 5 x 512^2 gradient, whose tensors are new on every call). True: built again.
@@ -2561,18 +2589,28 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     std::vector<double*>       f(fields, fields + nd);
     std::vector<const double*> gh;
     if (ghosts) gh.assign(ghosts, ghosts + 4 * nd);
-    if (u_ && f == u_->f && gh == u_->ghosts && steps == u_->steps) return false;
+    const bool capturing = is_capturing(s);
+    if (u_ && f == u_->f && gh == u_->ghosts && steps == u_->steps)
+    {
+        if (capturing) note_capture(s);
+        return false;
+    }
+    if (capturing) throw Error(3, "only the fields of the call before can be captured: solve them once outside a capture");
     // the ghost pass's list holds the subdomains that have ghosts: the same ones for a refill
     auto ghosted = [&](const std::vector<const double*>& v, int g) {
         return !v.empty() && (v[4 * g] || v[4 * g + 1] || v[4 * g + 2] || v[4 * g + 3]);
     };
-    bool refill = u_ && steps == u_->steps && !is_capturing(s);  // a capture would only record the copies
+    bool refill = u_ && steps == u_->steps && *u_->graphs == 0;
     for (int g = 0; g < nd && refill; ++g) refill = ghosted(gh, g) == ghosted(u_->ghosts, g);
     std::unique_ptr<UserLists> fresh;
     if (!refill)
     {
         drop_graphs();
         FPB_CUDA(cudaDeviceSynchronize());  // the lists may still be read by queued work
+        captured_.erase(std::remove_if(captured_.begin(), captured_.end(),
+                                       [](const std::unique_ptr<UserLists>& l) { return *l->graphs == 0; }),
+                        captured_.end());
+        captured_.reserve(captured_.size() + 1);
         fresh.reset(new UserLists());
     }
     UserLists& L = refill ? *u_ : *fresh;
@@ -2661,7 +2699,11 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     L.f      = f;
     L.ghosts = gh;
     L.steps  = steps;
-    if (fresh) u_ = std::move(fresh);
+    if (fresh)
+    {
+        if (u_ && *u_->graphs > 0) captured_.push_back(std::move(u_));
+        u_ = std::move(fresh);
+    }
     return !refill;
 }
 
@@ -2769,7 +2811,7 @@ template <typename TS> void BatchImpl<TS>::solve_graph(double* const* fields, co
     if (steps < 0 || steps > 64) throw Error(1, "steps must be in [0, 64]");
     const StreamOrder::Call call(&order, s);
     const bool              built = set_user_lists(fields, ghosts, steps, s);
-    if (lazy && (built || is_capturing(s)))
+    if ((lazy && built) || is_capturing(s))
     {
         run(steps, s);
         return;

@@ -153,7 +153,11 @@ int fp_composite_create(const fp_geometry* g, int m, double tol, int max_iter, i
 /* ConcatPoissonSolver2D::set_parameter (concat_solver2d.cpp:7-17). */
 int fp_composite_set_parameter(fp_composite* c, int m, double tol, int max_iter);
 /* ConcatPoissonSolver2D::solve: fields[d] (RHS in, solution out, in place); ghosts[4*d + face] are the
- * Variable2D ghost buffers (NULL = zero), length ny for x faces and nx for y faces. */
+ * Variable2D ghost buffers (NULL = zero), length ny for x faces and nx for y faces.
+ * On the spectral path this call, fp_composite_adjoint_f64 and fp_batch_solve may be captured into a CUDA graph
+ * (FP_DEVICE) after one call on the same fields and ghosts outside the capture; others give FP_ERR_UNSUPPORTED.
+ * The graph keeps solving the fields it was captured with, whatever the solver is called on later. The solver must
+ * outlive it, and its launches must be ordered after and before the solver's other calls by the caller. */
 int fp_composite_solve_f64(fp_composite* c, double* const* fields, const double* const* ghosts, int flags,
                            void* stream, fp_solve_info* info);
 /* The same problem by mixed-precision iterative refinement (no counterpart in the reference, which is
@@ -306,8 +310,9 @@ int fp_composite3d_destroy(fp_composite3d* c);
 typedef struct fp_batch fp_batch;
 #define FP_BATCH_F32 64          /* create flag: FP32 storage and arithmetic in the inner solves */
 #define FP_BATCH_NO_AUTOTUNE 128 /* create flag: keep the default launch shapes (no timing at creation) */
-#define FP_BATCH_GRAPH 256       /* solve flag: capture the launch sequence into a CUDA graph once per
-                                    (field pointers, steps) and replay it on later calls */
+#define FP_BATCH_GRAPH 256       /* solve flag: capture the launch sequence into a CUDA graph once per number of
+                                    steps and replay it on later calls; other fields, and ghosts on the same
+                                    subdomains, only change the lists it reads */
 /* problems[p].root is ignored (the reference's rule picks the root). */
 int fp_batch_create(const fp_geometry* problems, int n_problems, int flags, fp_batch** out);
 /* fields: device pointers (FP_DEVICE required), one per subdomain, problems back to back in creation

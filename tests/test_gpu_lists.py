@@ -109,3 +109,63 @@ def test_stream_handle_given_out_again():
     torch.cuda.synchronize()
     assert _same(torch, a, want_a) and _same(torch, b, want_b), second == first
     assert int(rt.cudaStreamDestroy(second)) == 0
+
+
+@pytest.mark.parametrize("form", ["solve", "adjoint", "batch", "batch_graph"])
+def test_captured_solve_keeps_its_fields(form):
+    """A caller's graph solves the fields it was captured with, also after calls on other fields, a second graph and the
+    end of the first; fields the solver has not seen cannot be captured."""
+    torch = torch_cuda()
+    g = W.cross(64, neumann_tips=True)
+
+    def make():
+        if form.startswith("batch"):
+            b = capi.Batch([g])
+            return lambda x: b.solve(x, steps=2, graph=form == "batch_graph")
+        c = capi.Composite(g, m=20, tol=1e-12, max_iter=100)
+        return getattr(c, form)
+
+    one, fresh = make(), make()
+    rhs = [_rhs(torch, g, k) for k in range(3)]
+    want = [_solved(torch, fresh, f) for f in rhs]
+    f = [[x.clone() for x in r] for r in rhs]
+
+    def refill():
+        for a, b in zip(f, rhs):
+            for x, y in zip(a, b):
+                x.copy_(y)
+
+    def captured(k):
+        one(f[k])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            one(f[k])
+        return graph
+
+    first = captured(0)
+    one(f[1])
+    one(f[1])
+    refill()
+    one(f[2])
+    first.replay()
+    torch.cuda.synchronize()
+    assert _same(torch, f[0], want[0]) and _same(torch, f[1], rhs[1]) and _same(torch, f[2], want[2])
+    second = captured(1)
+    refill()
+    second.replay()
+    first.replay()
+    one(f[2])
+    torch.cuda.synchronize()
+    assert all(_same(torch, a, b) for a, b in zip(f, want))
+    refused = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(refused):
+        with pytest.raises(capi.FpError):
+            one([x.clone() for x in f[0]])
+    torch.cuda.synchronize()
+    del first, refused
+    for k in (0, 2, 0, 2):
+        refill()
+        one(f[k])
+        second.replay()
+        torch.cuda.synchronize()
+        assert _same(torch, f[k], want[k]) and _same(torch, f[1], want[1])
