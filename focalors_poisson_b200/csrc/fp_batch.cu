@@ -1573,6 +1573,9 @@ private:
     void   edge_mv(const Segments& l, cudaStream_t s);
     void   build_ir_lists();
     void   note_capture(cudaStream_t s);
+    // One solve takes the fields without an assembly pass: the chase applies the hx^2 factor. FP64 rows only; FP32 ones
+    // would be rounded before they are scaled, and values whose transform exceeds 3e38 (1e38 on 64 x 64) would overflow.
+    bool   unassembled() const { return tile_ && std::is_same<TS, double>::value; }
     bool   set_user_lists(double* const* fields, const double* const* ghosts, int steps, cudaStream_t s);
     ResSeg res_seg(size_t g, double* r, const double* fs, const double* const* u_user);
     void   run(int steps, cudaStream_t s);
@@ -2681,7 +2684,7 @@ bool BatchImpl<TS>::set_user_lists(double* const* fields, const double* const* g
     }
     if (refill)
     {
-        if (ir || !tile_) L.assemble.refill(as, s);
+        if (ir || !unassembled()) L.assemble.refill(as, s);
         if (!ir)
         {
             L.ghost.refill(gs, s);
@@ -2767,7 +2770,7 @@ template <typename TS> void BatchImpl<TS>::add_norms(int first, cudaStream_t s)
 
 template <typename TS> void BatchImpl<TS>::run(int steps, cudaStream_t s)
 {
-    if (steps == 0 && tile_)  // the chase applies the hx^2 factor; only ghost values need a pass of their own
+    if (steps == 0 && unassembled())  // only ghost values need a pass of their own
     {
         const Segments& l = u_->ghost;
         if (l.n)
