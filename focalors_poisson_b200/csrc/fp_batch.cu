@@ -1255,11 +1255,14 @@ struct XList
         for (int k : {K_DD, K_ND, K_DN})
         {
             std::map<int, std::vector<size_t>> groups;  // -1: stage engine, -2: dense, else M of the register engine
+            long long                          rows = 0;  // of the launch that all dense runs would make
+            for (size_t i = 0; i < recs.size(); ++i)
+                if (kinds[i] == k && ps.tr[recs[i].plan]->dense) rows += recs[i].rows;
             for (size_t i = 0; i < recs.size(); ++i)
                 if (kinds[i] == k)
                 {
-                    const FftDesc& d = ps.tr[recs[i].plan]->fd;
-                    groups[d.eng == 1 ? d.M : d.eng == 3 ? -2 : -1].push_back(i);
+                    const DevTransform<T>& t = *ps.tr[recs[i].plan];
+                    groups[t.rule.product(rows) ? -2 : t.fd.eng == 1 ? t.fd.M : -1].push_back(i);
                 }
             for (auto& g : groups)
             {

@@ -62,20 +62,71 @@ __global__ void k_dense_tables(int kind, int inv, int n, int K, int C, int rows,
 }
 }  // namespace
 
-// Where the line lies (us for 4.2 M cells in place, FFT against product, forward / inverse): FP64 DD 256: 72 / 63, 320:
-// 83 / 97; ND 224: about 100 / 84, 256: 93, 108 / 105; NN 96: 55, 60 / 48, 41, 128: 43, 48 / 45, 39, 144: 44, 53 / 62,
-// 56; PP 144: 86, 92 / 69, 60, 192: 61, 64 / 97, 87. Well below it the product wins by more (DD 128: 97 / 38, 64: 176 /
-// 27). FP32 rows keep FP64 arithmetic here, so their line is lower: DD 192: 70 / 51, 256: 46 / 61; ND 192: 90, 106 / 75,
-// 75. 131 k cells: DD 256 13.9 / 8.2, 128 9.2 / 5.8, ND 192 13, 15 / 11, 11.
-int dense_limit(int kind, bool f32)
+// Where the lines lie, by row length n, rows of a run, storage of the FFT it replaces and whether that FFT is one of
+// its own length (7-smooth n + 1, n or 2 n + 1: direct) or a convolution of twice the length, two to three times as
+// dear. Time of the product over the FFT's, forward + inverse, in place:
+//   rows                   128  1024  2048  3072  4736  4768  8192 32768
+//   FP64 DD  95 direct     .87   .97   .97  1.32   .83   .97   .72   .67
+//   FP64 DD 127 direct     .90  1.00  1.06  1.42  1.00  1.17   .89   .86
+//   FP64 DD 159 direct    1.14  1.27  1.52  1.79  1.23  1.57  1.13  1.09
+//   FP64 DD 192            .75   .80   .99  1.02   .69   .96   .66   .58
+//   FP64 DD 256            .53   .75  1.19  1.26   .83  1.20   .95   .78
+//   FP64 NN  64 direct     .83   .82   .82   .80   .66   .77   .58   .55
+//   FP64 NN  96 direct     .91   .92  1.04  1.38   .82  1.01   .74   .72
+//   FP64 PP  60 direct     .87   .82   .55   .52   .50   .55   .39   .34
+//   FP64 PP  96 direct    1.16  1.06   .84  1.11   .72   .89   .61   .59
+//   FP64 PP 144 direct    1.32  1.33  1.05  1.19   .87  1.11   .75   .72
+//   FP64 DN 121 direct     .73   .79  1.05  1.27   .68   .97   .74   .75
+//   FP64 DN 187 direct    1.24  1.33  2.00  1.91  1.23  1.99  1.38  1.35
+//   FP64 DN 192            .69   .76  1.04   .91   .62  1.04   .70   .62
+//   FP64 DN 224            .50   .86  1.24  1.13   .77  1.26   .85   .76
+//   FP32 DD 127 direct    1.01  1.08  1.13  1.57  1.23  1.23  1.03   .93
+//   FP32 DD 192            .85   .89  1.14  1.21   .96  1.10   .82   .69
+//   FP32 PP 144 direct    1.36  1.40  1.44  1.21   .96  1.16   .82   .78
+//   FP32 DN 192            .89   .95  1.36  1.26  1.00  1.38   .97   .80
+// The steps are waves of 32-row tiles, 148 and 296 of them (4736 and 9472 rows), and the change of launch shape at
+// 2560 or 3200 rows. Where they cross 1 the FFT takes the rows between, one range per band; beside it up to a tenth, at
+// a few lengths two or three in the first rows of a wave, is left. FP32 rows keep FP64 arithmetic in the product and have
+// the faster FFT, so their lines are lower.
+namespace
 {
-    switch (kind)
-    {
-        case K_DD: return f32 ? 224 : 256;
-        case K_NN: return 96;
-        case K_PP: return 144;
-        default: return f32 ? 192 : 224;
-    }
+constexpr int kNever = INT_MAX;
+struct DenseBand  // row lengths up to `last` (from the band before)
+{
+    int last, from, to;  // FFT for `from` <= rows < `to`
+};
+using Bands = std::vector<DenseBand>;
+const Bands& dense_bands(int kind, bool direct, bool f32)
+{
+    // [FP64 / FP32][family][convolution / direct]
+    static const Bands b[2][4][2] = {
+        {{{{144, 0, 0}, {199, 2048, 3584}, {256, 1536, 8192}}, {{63, 0, 0}, {96, 2048, 3584}, {127, 2048, 7168}}},
+         {{{96, 0, 0}}, {{64, 0, 0}, {96, 2048, 3584}}},
+         {{{199, 0, 0}, {224, 2048, 3584}},
+          {{64, 0, 0}, {127, 2048, 3584}, {190, 0, kNever}, {224, 1024, kNever}}},
+         {{{144, 0, 0}}, {{60, 0, 0}, {126, 0, 2048}, {144, 0, 7168}}}},
+        {{{{144, 0, 0}, {199, 1536, 6144}, {224, 1536, kNever}},
+          {{63, 0, 0}, {96, 2560, 4736}, {127, 1536, 12288}}},
+         {{{96, 0, 0}}, {{64, 0, 0}, {96, 1024, 5632}}},
+         {{{128, 0, 0}, {144, 2048, 14208}, {175, 1536, kNever}, {192, 1536, 8192}},
+          {{64, 0, 0}, {80, 2048, 7168}, {121, 1536, 14208}}},
+         {{{144, 0, 0}}, {{60, 0, 0}, {126, 0, 3200}, {144, 0, 7168}}}}};
+    const int family = kind == K_DD ? 0 : kind == K_NN ? 1 : kind == K_PP ? 3 : 2;
+    return b[f32][family][direct];
+}
+}  // namespace
+
+DenseRule dense_rule(int kind, int n, bool f32)
+{
+    DenseRule r;
+    for (const DenseBand& b : dense_bands(kind, fft_direct(fft_length(kind, n)), f32))
+        if (n <= b.last)
+        {
+            r.from = b.from;
+            r.to   = b.to == kNever ? LLONG_MAX : b.to;
+            break;
+        }
+    return r;
 }
 
 DensePlan::DensePlan(int kind_, int n_) : kind(kind_), n(n_)
@@ -162,7 +213,10 @@ DenseShape dense_shape(int kind, const std::vector<DenseLoad>& loads)
     auto smem = [&](int c) { return (size_t)dense_smem(fold, maxK, kCfgBM[c], kCfgBN[c]) * sizeof(double); };
     DenseShape sh;
     sh.cfg = kSmall;
-    if (rows >= 100LL * kCfgBM[0])  // the column tile with the least work, padding included
+    // From 80 tiles of 32 rows on (100 where the products are narrow), the column tile with the least work, padding
+    // included. us, large / small tiles, FP64: 2560 rows DD 120 10.1 / 8.1, DD 160 14.2 / 15.9; 3200 rows DD 64 5.6 / 5.1,
+    // DD 128 9.7 / 10.8, DD 160 14.3 / 17.6, ND 192 19.4 / 24.2.
+    if (rows >= (maxC <= 64 ? 100LL : 80LL) * kCfgBM[0])
     {
         double best = 0;
         for (int c = 0; c < kSmall; ++c)

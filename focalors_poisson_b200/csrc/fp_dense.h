@@ -7,8 +7,8 @@
 namespace fpb
 {
 
-// Row length up to which a family runs as a dense product.
-int dense_limit(int kind, bool f32);
+// When rows of length n of a family run as dense products; f32: instead of FP32 FFTs.
+DenseRule dense_rule(int kind, int n, bool f32);
 
 // Tables of one family and row length; both directions.
 struct DensePlan

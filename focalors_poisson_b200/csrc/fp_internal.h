@@ -5,6 +5,7 @@
 #include "fp_plan.h"
 #include "fp_transform.cuh"
 
+#include <climits>
 #include <cuda_runtime.h>
 
 #include <memory>
@@ -180,6 +181,14 @@ private:
 };
 
 struct DensePlan;     // fp_dense.h
+// Runs of `from` to `to` - 1 rows of a transform go by FFT, the others as dense products (dense_rule, fp_dense.cu).
+struct DenseRule
+{
+    long long from = 0, to = LLONG_MAX;  // never a product
+    bool      any() const { return from > 0 || to < LLONG_MAX; }
+    bool      always() const { return from >= to; }
+    bool      product(long long rows) const { return rows < from || rows >= to; }
+};
 struct ChaseTileTab;  // fp_chase_tile.cuh
 
 // Device-resident plan for one transform family at one row length and precision.
@@ -196,7 +205,8 @@ template <typename T> struct DevTransform
     size_t  smem    = 0;
     int     gctas   = 0;
     long long gstride = 0;
-    std::shared_ptr<DensePlan> dense;  // short rows: a product with the matrix (fd.eng = 3, no FFT plan)
+    std::shared_ptr<DensePlan> dense;  // short rows: a product with the matrix for the row counts of `rule`
+    DenseRule                  rule;   // always a product: no FFT plan (fd.eng = 3)
 
     // allow_register false: keep the plan on the stage engine (callers that launch plans of several
     // lengths with one CTA shape). allow_global: rows whose FFT buffer exceeds a CTA's shared memory run

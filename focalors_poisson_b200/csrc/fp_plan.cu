@@ -147,6 +147,8 @@ int fft_length(int kind, int n)
     }
 }
 
+bool fft_direct(int L) { return L == 1 || !radices(L).empty(); }
+
 FftWindow fft_window(int kind, int n, bool inverse)
 {
     if (kind == K_ND && inverse) return FftWindow{1, 2 * n, 1, n};  // herm_input 1..2n; outputs X_{j+1}

@@ -46,6 +46,8 @@ int kind_of(int bc_neg, int bc_pos);  // -1 if unsupported
 
 // Length of the complex FFT each family's device transform runs (fp_transform.cuh).
 int fft_length(int kind, int n);
+// Whether a DFT of length L runs as radix stages of its own length (7-smooth), else as a convolution.
+bool fft_direct(int L);
 
 // Inputs a transform reads and outputs it keeps, for Bluestein's windowed convolution (fp_fft.cuh).
 struct FftWindow

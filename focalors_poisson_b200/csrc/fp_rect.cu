@@ -123,9 +123,10 @@ DevTransform<T>::DevTransform(int kind_, int n_, bool allow_register, bool allow
 {
     if (n < 2) throw Error(1, "row length must be at least 2");
     if (kind == K_PP && (n % 2)) throw Error(1, "periodic transform needs an even length");
-    if (allow_register && n <= dense_limit(kind, std::is_same<T, float>::value))
+    if (allow_register) rule = dense_rule(kind, n, std::is_same<T, float>::value);
+    if (rule.any()) dense.reset(new DensePlan(kind, n));
+    if (rule.always())
     {
-        dense.reset(new DensePlan(kind, n));
         fd.eng = fd_inv.eng = 3;
         return;
     }
@@ -219,7 +220,7 @@ template <typename TIO>
 void DevTransform<T>::run_io(const TIO* in, TIO* out, long long rows, bool inverse, cudaStream_t s) const
 {
     if (rows > (long long)INT_MAX) throw Error(3, "more than 2^31 rows in one transform call");
-    if (dense)
+    if (rule.product(rows))
     {
         const bool f32 = std::is_same<TIO, float>::value;
         dense_rows(*dense, inverse, in, out, rows, f32, f32 ? DENSE_F32 : DENSE_F64, s);

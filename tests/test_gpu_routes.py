@@ -1,11 +1,14 @@
 """Calls at the sizes and values where the library changes the way it takes: both ways must give the same."""
+import numpy as np
 import pytest
 
-from gpu_util import torch_cuda
+from gpu_util import rel_max, torch_cuda
+from oracle import fp_oracle as O
 from focalors_poisson_b200 import capi
 from focalors_poisson_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
+PAIRS = {"DD": (0, 0), "NN": (1, 1), "ND": (1, 0), "DN": (0, 1), "PP": (2, 2)}
 
 
 def test_fp32_rows_are_scaled_before_they_are_rounded():
@@ -20,3 +23,38 @@ def test_fp32_rows_are_scaled_before_they_are_rounded():
     top = max(float(y.abs().max()) for y in want)
     for x, y in zip(got, want):
         assert float((x / 1e38 - y).abs().max()) <= 1e-4 * top
+
+
+@pytest.mark.parametrize("kind,ny", [("DD", 63), ("DD", 95), ("DD", 127), ("DD", 128), ("DD", 134), ("DD", 199), ("DD", 224),
+                                     ("DD", 256), ("NN", 64), ("NN", 96), ("NN", 95), ("PP", 60), ("PP", 64), ("PP", 126),
+                                     ("PP", 128), ("PP", 144), ("ND", 67), ("ND", 122), ("ND", 157), ("ND", 224),
+                                     ("DN", 94), ("DN", 175), ("DN", 192), ("DN", 200)])
+def test_product_and_fft_rows_vs_oracle(kind, ny):
+    """Row counts on both sides of every line between the dense product and the FFT, and of the change of launch shape;
+    row lengths at the ends of the bands. In place, FP64 at 1e-13 and FP32 rows at 2e-5 as for the other transforms."""
+    torch = torch_cuda()
+    f = np.random.default_rng(ny).standard_normal((12288, ny))
+    for inv in (False, True):
+        ref = (O.transform_inverse if inv else O.transform_forward)(kind, f)
+        for rows in (1535, 1536, 2047, 2048, 2559, 2560, 3072, 3200, 3584, 5632, 7167, 7168, 12287, 12288):
+            for dtype, bound in ((torch.float64, 1e-13), (torch.float32, 2e-5)):
+                t = torch.tensor(f[:rows], device="cuda", dtype=dtype)
+                capi.transform(*PAIRS[kind], t, inverse=inv, out=t)
+                assert rel_max(t.double().cpu().numpy(), ref[:rows]) <= bound, (kind, ny, rows, inv, dtype)
+
+
+def test_batched_lists_by_product_and_by_fft():
+    """1, 2 and 10 crosses of 256 x 256 are 1280, 2560 and 12800 rows a launch: product, FFT, product. Every problem's
+    solution against the others' (1e-11 as for the other composite solves; FP32 in three refinement steps 1e-10)."""
+    torch = torch_cuda()
+    g = W.cross(256)
+    f = [torch.tensor(x, device="cuda") for x in W.gaussian_rhs(g, 3)]
+    for precision, steps, bound in (("f64", 0, 1e-11), ("f32", 3, 1e-10)):
+        want = None
+        for count in (1, 2, 10):
+            got = [x.clone() for _ in range(count) for x in f]
+            capi.Batch([g] * count, precision=precision).solve(got, steps=steps, sync=True)
+            want = want or got
+            top = max(float(x.abs().max()) for x in want)
+            for k, x in enumerate(got):
+                assert float((x - want[k % 5]).abs().max()) <= bound * top, (precision, count, k)
