@@ -27,6 +27,8 @@
 
 #include "fp_common.cuh"
 
+#include <climits>
+
 namespace fpb
 {
 
@@ -43,6 +45,27 @@ inline int tile_rows(int nx)
     for (int R : {16, 8, 4})
         if ((R < 16 || nx > 512) && (nx + R - 1) / R * (R - 1) <= nx) return R;
     return 0;
+}
+
+// Columns (fields x wavenumbers) up to which the one-pass kernel is the faster one on short columns. Most of a tile's
+// lanes are idle there (nx = 8 is one chunk: 8 threads of a warp), which many columns pay for, while one thread per
+// column (k_chase) is a chain of 2 nx steps that hides behind other columns; with periodic x it reads two more tables.
+// us, sequential / one-pass, DD: 64 columns nx 3 2.2 / 2.5, 8 3.4 / 3.0, 16 5.3 / 3.3; 32768 columns 8 3.7 / 5.7, 16 5.7 /
+// 5.9, 24 7.8 / 5.7; 262144 columns 8 9 / 23, 16 16 / 24, 24 24 / 25, 32 32 / 28; 127000 columns 33 16 / 24, 40 17 / 19.
+inline long long tile_columns(int nx, bool periodic)
+{
+    struct Line
+    {
+        int       last;
+        long long open, per;
+    };
+    constexpr long long never = LLONG_MAX;
+    static const Line lines[] = {{4, 0, 24576},         {8, 8192, 32768},       {13, 24576, 65536},   {16, 32768, 196608},
+                                 {20, 49152, 98304},    {24, 131072, never},    {27, 98304, never},   {32, never, never},
+                                 {34, 65536, 98304},    {41, 98304, never}};
+    for (const Line& l : lines)
+        if (nx <= l.last) return periodic ? l.per : l.open;
+    return never;
 }
 
 // The systems of one field: chunk layout and tables (chase_tile_tables builds them).

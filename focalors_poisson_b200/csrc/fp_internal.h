@@ -239,6 +239,7 @@ template <typename T> struct DevRect
     DevBuf                           sep_cp, sep_iden;          // separator-system Thomas factors [p][j]
     int                              sep_pmax = 0;              // rows of those tables
     bool                             tiled    = false;          // one-pass chase (fp_chase_tile.cuh): FP64, nx <= 4096
+    long long                        seq_from = LLONG_MAX;      // columns from which the sequential sweep runs instead
     int                              tile_R = 0, tile_P = 0, tile_e = 0, tile_types = 1;  // its chunks
     DevBuf                           tile_cq, tile_ends, tile_d, tile_cp, tile_iden, tile_v, tile_ib;
     mutable DevBuf                   scratch;                   // partition chase scratch (per batch)

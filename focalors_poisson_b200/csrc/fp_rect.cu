@@ -520,14 +520,15 @@ template <typename T> void DevRect<T>::build_chase_tables(const std::vector<doub
             tile_v  = upload(t.v);
             tile_ib = upload(t.ib);
         }
-        tile_P = t.P;
-        tile_e = t.e;
+        tile_P   = t.P;
+        tile_e   = t.e;
+        seq_from = tile_columns(nx, xp);
     }
-    if (tiled) return;  // the singular wavenumbers' recursion needs no table
+    if (tiled && seq_from == LLONG_MAX) return;  // the singular wavenumbers' recursion needs no table
     std::vector<double> c;
     chase_table(nx, ny, d, !xp && bc[XNEG] == BC_NEUMANN, !xp && bc[XPOS] == BC_NEUMANN, c);
     ctab = upload(convert<T>(c));
-    if (chunked)
+    if (chunked && !tiled)
     {
         std::vector<double> pc, pg, ph, pe;
         partition_tables(ny, d, bc[XNEG] == BC_NEUMANN, pc, pg, ph, pe);
@@ -574,7 +575,7 @@ template <typename T> long long DevRect<T>::chase_scratch_elems(long long batch)
 template <typename T> void DevRect<T>::chase(T* f, long long batch, T* scr, cudaStream_t s) const
 {
     if constexpr (std::is_same<T, double>::value)
-        if (tiled)
+        if (tiled && batch * ny < seq_from)
         {
             const ChaseTileTab t = tile_tab(nx);
             const int skip = singular ? ny - sing_from : 0;
@@ -588,7 +589,7 @@ template <typename T> void DevRect<T>::chase(T* f, long long batch, T* scr, cuda
             }
             return;
         }
-    if (!chunked)
+    if (!chunked || tiled)
     {
         const long long nthreads = batch * ny;
         const int       block    = 128;

@@ -58,3 +58,24 @@ def test_batched_lists_by_product_and_by_fft():
             top = max(float(x.abs().max()) for x in want)
             for k, x in enumerate(got):
                 assert float((x - want[k % 5]).abs().max()) <= bound * top, (precision, count, k)
+
+
+@pytest.mark.parametrize("nx", [3, 4, 7, 8, 13, 16, 20, 24, 27, 34, 41])
+def test_one_pass_and_sequential_columns(nx):
+    """Many short columns take one thread each, few the one-pass chase: field counts on both sides of every line between
+    them, against the same fields solved 32 at a time. Every x pair, and systems without a Dirichlet face. 1e-11 as for the
+    other rectangle solves."""
+    torch = torch_cuda()
+    ny = 64
+    f = torch.tensor(np.random.default_rng(nx).standard_normal((3072, nx, ny)), device="cuda")
+    for bc in ((0, 0, 0, 0), (1, 0, 0, 0), (0, 1, 0, 0), (1, 1, 0, 0), (2, 2, 0, 0), (1, 1, 1, 1), (2, 2, 1, 1)):
+        one = capi.Rect(nx, ny, 0.05, 0.07, bc)
+        want = f.clone()
+        for part in want.split(32):
+            one.solve(part)
+        top = float(want.abs().max())
+        for columns in (8192, 24576, 32768, 49152, 65536, 98304, 131072, 196608):
+            for fields in (columns // ny - 1, columns // ny):
+                got = f[:fields].clone()
+                one.solve(got)
+                assert float((got - want[:fields]).abs().max()) <= 1e-11 * top, (bc, columns, fields)
