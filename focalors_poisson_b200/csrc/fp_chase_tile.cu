@@ -44,9 +44,10 @@ template <int W, int R> void launch(double* f, long long batch, int skip, const 
 
 }  // namespace
 
-// Tile width: 8 wavenumbers (64-byte row pieces) while that keeps a CTA at 512 threads, else 4 (32 bytes, one
-// sector): with 512 threads of 64 registers two tiles share an SM. Before the paired factors 2048 x 2048 took
-// 27.5 us at 4, 29.7 us at 8, and 1000 x 1500 10.1 us at 4, 11.6 us at 8, 12.8 us at 16.
+// Tile width: 8 wavenumbers (64-byte row pieces) with 8-row chunks, 4 (32 bytes, one sector) with 16-row ones, whose CTA
+// is then 512 threads of 64 registers at 2048 rows, so that two tiles share an SM. us at W = 4 / 8 / 16: 8-row chunks 256 x
+// 256 3.0 / 3.1 / 4.0, 256 x 8192 10.1 / 8.4 / 9.7; 16-row chunks 1000 x 1000 6.7 / 6.3 / 10, 1280 x 1280 11.1 / 13.4,
+// 1536 x 1536 13.9 / 15.8, 2048 x 2048 21.6 / 21.1, 2048 x 512 7.2 / 11.
 void launch_chase_tile(double* f, long long batch, int skip, const ChaseTileTab& t, cudaStream_t s)
 {
     switch (t.R)

@@ -1,9 +1,9 @@
 // One-pass partition chase: the Thomas solves along x of W neighbouring wavenumbers by one CTA that holds all
 // their rows in registers, so that a field is read once and written once.
 //
-// Rows are cut into P chunks, the first e of R rows and the others of R - 1 (so any nx but a few below 13 divides,
-// tile_rows), thread (p, w) = (threadIdx.x / W, threadIdx.x % W) owns chunk p of wavenumber j = tile W + w. The last row of a chunk
-// is its separator B_p; the rows before it satisfy  x_int = z_p - B_{p-1} g - B_p h,  z_p = T^-1 f_int,
+// Rows are cut into P chunks, the first e of R rows and the others of R - 1 (any nx up to 4096 but 2 and 5 divides so,
+// tile_rows); thread (p, w) = (threadIdx.x / W, threadIdx.x % W) owns chunk p of wavenumber j = tile W + w. The last row
+// of a chunk is its separator B_p; the rows before it satisfy  x_int = z_p - B_{p-1} g - B_p h,  z_p = T^-1 f_int,
 // g = T^-1 e_first, h = T^-1 e_last, and the separators a tridiagonal system of size P whose Thomas factors
 // depend on the wavenumber only and are tabulated:
 //   -g_last B_{p-1} + (d - h_last - g'_first) B_p - h'_first B_{p+1} = f_sep - z_last - z'_first
@@ -18,7 +18,7 @@
 // The result equals the sequential Thomas solve (chasing_method_base.cpp:24-52) and, for periodic x, the
 // Sherman-Morrison solve (:178-197) up to round-off.
 //
-// What bounds it: one read and one write of the field (L2 or HBM); 2048 x 2048 in 23.7 us, 2.8 TB/s (the three-pass
+// What bounds it: one read and one write of the field (L2 or HBM); 2048 x 2048 in 21.7 us, 3.1 TB/s (the three-pass
 // form: 48 us), 256 x 65536 in 81 us, 3.3 TB/s, 1000 x 1500 in 8.6 us (sequential sweep: 764 us); the load, compute
 // and store phases of the few tiles an SM holds overlap little. At R = 16 the kernel stays at 64 registers, so that an
 // SM holds 1024 threads of tiles, and the dependent chains at 15 steps. Only the last interior row of a chunk is
@@ -36,9 +36,10 @@ constexpr int kTileThreads = 1024;  // largest CTA: kTileThreads / 4 chunks
 constexpr int kTileMaxRows = kTileThreads / 4 * 16;
 
 // Rows of the longer chunks for nx rows, whose chunks of R and R - 1 rows must add up to nx; 0 where none does (nx = 2
-// and 5) or nx is beyond one CTA. 16 above 512 rows; 8 below, where a field gives few tiles and the pass is a chain
-// of latencies (graph replays before the paired factors, 128 x 128 / 384 x 384 / 96 x 11520 periodic: 3.2 / 4.0 / 5.8
-// us against 4.8 / 4.4 / 8.3 us at R = 16; 2048 x 2048: 34.8 us against 27.5 us).
+// and 5) or nx is beyond one CTA. 16 above 512 rows; 8 below, where a field gives few tiles and the pass is a chain of
+// latencies. us at (R, W) = (8, 8) / (16, 4) / (16, 8), graph replays: 128 x 128 2.7 / 3.7 / 3.5, 512 x 512 4.2 / 3.8 /
+// 4.2, 1024 x 512 7.4 / 4.7 / 6.1, 2048 x 512 - / 7.2 / 11; with more tiles (16, 8) is the better one from 192 to 1024
+// rows, which the rule does not use: 384 x 8192 14.7 / 13.9 / 11.3, 512 x 8192 18.8 / 18.1 / 14.3, 1024 x 2048 14 / 11 / 9.
 inline int tile_rows(int nx)
 {
     if (nx > kTileMaxRows) return 0;
@@ -98,7 +99,6 @@ template <int W, bool REV>
 __device__ __forceinline__ double tile_scan(double a, double b, double2* tw)
 {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, w = lane % W;
-    // W = 32: a warp holds one chunk
 #pragma unroll
     for (int o = W; o < 32; o <<= 1)
     {
@@ -126,8 +126,9 @@ __device__ __forceinline__ double tile_scan(double a, double b, double2* tw)
 // One tile. IO: in(i, j) the address of a right-hand side (rows ny apart); stage() loads what mods() needs into shared
 // memory (a barrier follows); mods(y, fsep, lng, i0, li, j) turns the thread's values (interior rows i0 + r, separator
 // row i0 + li) into right-hand sides; store() says whether the solution is written, to out(i, j), or handed to
-// take(y, x, lng, p, i0, li, j, on) by all threads of a warp together (interior rows and separator, `on` where valid). skip: wavenumbers from ny - skip on are left alone. The tile's
-// wavenumbers are tile W .. tile W + W - 1; blockDim.x a multiple of 32 of at least P W.
+// take(y, x, lng, p, i0, li, j, on) by all threads of a warp together (interior rows and separator, `on` where valid).
+// skip: wavenumbers from ny - skip on are left alone. The tile's wavenumbers are tile W .. tile W + W - 1; blockDim.x a
+// multiple of 32 of at least P W.
 template <int W, int R, typename IO>
 __device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int skip, const IO& io, double* sm)
 {

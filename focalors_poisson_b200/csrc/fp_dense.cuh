@@ -316,8 +316,7 @@ __global__ void __launch_bounds__(WM* WN * 32, 2)
         if (in32) fill_rows(static_cast<const float*>(sg.in) + base);
         else fill_rows(static_cast<const double*>(sg.in) + base);
     }
-    else if (in32) fill_cols(static_cast<const float*>(sg.in) + base);
-    else fill_cols(static_cast<const double*>(sg.in) + base);
+    else fill_cols(static_cast<const double*>(sg.in) + base);  // the middle axis of FP64 fields
     if (CS > 1)  // every CTA of the cluster has read the rows before any of them stores
     {
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
