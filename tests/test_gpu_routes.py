@@ -79,3 +79,32 @@ def test_one_pass_and_sequential_columns(nx):
                 got = f[:fields].clone()
                 one.solve(got)
                 assert float((got - want[:fields]).abs().max()) <= 1e-11 * top, (bc, columns, fields)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_bad_value_stays_in_its_row_field_and_problem(bad):
+    """One bad value spoils its own row of a dense transform (tiles of 32 and of 8 rows), its own field of a rectangle or
+    box solve and its own problem of a batch; everything else is what it is without it, bit for bit."""
+    torch = torch_cuda()
+    gen = torch.Generator(device="cuda").manual_seed(1)
+
+    def check(run, shape, item):
+        f = torch.randn(shape, generator=gen, dtype=torch.float64, device="cuda")
+        g = f.clone()
+        g[item].view(-1)[g[item].numel() // 3] = bad
+        run(f)
+        run(g)
+        torch.cuda.synchronize()
+        keep = torch.ones(shape[0], dtype=torch.bool, device="cuda")
+        keep[item] = False
+        assert torch.equal(f[keep], g[keep]) and bool(torch.isfinite(f).all()) and not bool(torch.isfinite(g[item]).all())
+
+    for kind, ny, rows in (("DD", 128, 4000), ("NN", 64, 100), ("PP", 144, 8000), ("ND", 96, 37)):
+        for inv in (False, True):
+            check(lambda x: capi.transform(*PAIRS[kind], x, inverse=inv, out=x), (rows, ny), rows // 2)
+    for nx, ny, bc in ((64, 96, (0, 0, 0, 0)), (600, 40, (1, 0, 0, 0)), (100, 64, (2, 2, 0, 0)), (8, 64, (0, 0, 0, 0))):
+        check(capi.Rect(nx, ny, 0.05, 0.07, bc).solve, (3, nx, ny), 1)
+    check(capi.Rect3D(16, 32, 24, 0.05, 0.07, 0.06, (0, 0, 0, 0, 2, 2)).solve, (3, 16, 32, 24), 1)
+    g = W.cross(64)
+    b = capi.Batch([g] * 3)
+    check(lambda x: b.solve([x[p, d] for p in range(3) for d in range(5)], sync=True), (3, 5, 64, 64), 1)
