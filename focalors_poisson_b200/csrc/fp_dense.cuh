@@ -8,7 +8,7 @@
 //                    two outputs of a frequency are s1 (ta S + tb C)  (and the transpose for the inverse)
 //   ND, DN           no reflection symmetry: the full matrix, its columns in two halves
 // So a row needs n^2 (ND, DN: 2 n^2) operations, the fast transform of the awkward lengths of these families
-// (n + 1, 2 n + 1) several hundred n: dense_limit says where the product stops being the faster one.
+// (n + 1, 2 n + 1) several hundred n: dense_rule says where the product is the faster one.
 //
 // A CTA takes BM rows whole into shared memory (folded), so that rows may be transformed in place, then runs over
 // column tiles, streaming the table through a cp.async ring while eight warps accumulate in registers.
