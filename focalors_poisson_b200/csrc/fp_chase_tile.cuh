@@ -137,7 +137,7 @@ __device__ __forceinline__ void chase_tile(const ChaseTileTab& t, int tile, int 
     const int     w   = tid % W, p = tid / W, P = t.P, ny = t.ny;
     const int     j0  = tile * W + w;
     const bool    act = p < P && j0 < ny - skip;
-    const int     j   = j0 < ny ? j0 : 0;  // idle lanes read column 0 and store nothing
+    const int     j   = min(j0, ny - 1);  // idle lanes read their own tile's last column (another's is being stored)
     double2*      cs  = reinterpret_cast<double2*>(sm);  // [2][Ri][W]
     double2*      tw  = cs + 2 * Ri * W;                 // warps' compositions, forward and backward
     double2*      tw2 = tw + (n / 32) * W;
