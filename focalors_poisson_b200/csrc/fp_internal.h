@@ -141,9 +141,10 @@ inline bool is_capturing(cudaStream_t s)
     return cs != cudaStreamCaptureStatusNone;
 }
 
-// Queues the calls on one object's buffers one after the other, whatever streams they come on: each waits for an event
-// recorded at the end of the one before (an equal stream handle proves no order, it may have been destroyed with work
-// queued and given out again). A call being captured is left out; its graph's launches are the caller's to order.
+// Queues the calls on one object's buffers one after the other, whatever streams they come on: a call on another stream
+// than the one before waits for an event recorded at its end. Streams are told apart by their ids (an equal handle proves
+// no order, it may have been destroyed with work queued and given out again); the wait costs a small solve 1 us of 69. A
+// call being captured is left out; its graph's launches are the caller's to order.
 class StreamOrder
 {
 public:
@@ -161,8 +162,11 @@ public:
         Call(StreamOrder* o, cudaStream_t s) : o_(o && !is_capturing(s) ? o : nullptr), s_(s)
         {
             if (!o_) return;
+            unsigned long long id = 0;
+            FPB_CUDA(cudaStreamGetId(s_, &id));
             if (!o_->e_) FPB_CUDA(cudaEventCreateWithFlags(&o_->e_, cudaEventDisableTiming));
-            else FPB_CUDA(cudaStreamWaitEvent(s_, o_->e_, 0));
+            else if (id != o_->id_) FPB_CUDA(cudaStreamWaitEvent(s_, o_->e_, 0));
+            o_->id_ = id;
         }
         ~Call()
         {
@@ -177,7 +181,8 @@ public:
     };
 
 private:
-    cudaEvent_t e_ = nullptr;
+    cudaEvent_t        e_  = nullptr;
+    unsigned long long id_ = 0;  // of the last call's stream
 };
 
 struct DensePlan;     // fp_dense.h
